@@ -262,14 +262,12 @@ tomo_status tomo_batch_set_priority(tomo_batch* b, int32_t priority);
  * Members' own streams must be idle at each iteration, as with the batch's own stream. */
 tomo_status tomo_batch_set_stream(tomo_batch* b, void* stream);
 /* Persistent launches (no counterpart in the reference; default off): each forward phase
- * is one launch per CTA size (256 threads up to 512 detector columns, 512 above) and each
- * backprojection phase one launch per storage type and rule set, of resident CTAs that
- * take work items from a device list, longest first, through an atomic cursor.  Off: one
- * launch per kernel variant with a CTA per item, which measured faster on GB300 (64
- * heterogeneous series: 0.97 against 0.85-0.88 T voxel-updates/s).  Results are bitwise
+ * is one launch, and each backprojection phase one launch per storage type and rule set, of
+ * resident CTAs that take work items from a device list, longest first, through an atomic
+ * cursor.  Off: one launch per kernel variant with a CTA per item.  Results are bitwise
  * the same.  on: 0 off, 1 on; for tuning, a sum of 2 (forward phase persistent), 4
  * (backprojection persistent), 8 (lists in plan order instead of longest first) and 16
- * (launches of a phase one after another instead of side by side). */
+ * (backprojection launches of a phase one after another instead of side by side). */
 tomo_status tomo_batch_set_persistent(tomo_batch* b, int32_t on);
 /* Replaces the membership (n handles). */
 tomo_status tomo_batch_set(tomo_batch* b, tomo_projector* const* members, int32_t n);

@@ -4,9 +4,10 @@
 // tables and options) and runs one OS-SART iteration of all of them together:
 // for every update index s, one forward-projection launch per kernel variant
 // covers update s of every member that has one (each CTA reads its
-// {descriptor, tilt group, row} work item), one batched residual reduction
-// follows, and one backprojection launch covers all members' tiles.  Optionally
-// (tomo_batch_set_persistent) each phase is one persistent launch per CTA size
+// {descriptor, tilts and window, rows, segment} work item) and one closing pass
+// adds the segments, one batched residual reduction follows, and one
+// backprojection launch covers all members' tiles.  Optionally
+// (tomo_batch_set_persistent) the forward launches of a phase are one persistent launch
 // instead: resident CTAs take items from a list, longest first, through an
 // atomic cursor, and the launches of a phase run side by side.  The
 // per-member descriptors and work lists are rebuilt only when the membership
@@ -69,6 +70,13 @@ struct tomo_batch {
         size_t smem;
         int off, n;
     };
+    // row-vector form: projector items of piece c (the tilts whose segment sums fit the
+    // members' scratch) of update s; zc 0: the closing pass of the piece
+    struct FprSeg {
+        int s, c, zc, eb;
+        size_t smem;
+        int off, n, cursor;  // cursor >= 0: a persistent launch
+    };
     struct BpSeg {
         int s;
         bool sanitize, pos;
@@ -85,14 +93,9 @@ struct tomo_batch {
     std::vector<VolSeg> vol_segs;
     VolJob* d_vjobs = nullptr;
     size_t cap_vjobs = 0;
-    // persistent launches: one per (s, block size, chunk depth) for the forward phase and
-    // per (s, flags, storage type, row pairs) for the backprojection; cursor: its slot of
-    // d_cursor, zeroed at the start of every iteration
-    struct FpPSeg {
-        int s, nt, zc;
-        size_t smem;
-        int off, n, cursor, grid;
-    };
+    // persistent launches: one per (s, piece) for the forward phase and per (s, flags,
+    // storage type, row pairs) for the backprojection; cursor: its slot of d_cursor, zeroed
+    // at the start of every iteration
     struct BpPSeg {
         int s;
         bool sanitize, pos;
@@ -103,7 +106,8 @@ struct tomo_batch {
     std::vector<FpSeg> fp_segs;
     std::vector<BpSeg> bp_segs;
     std::vector<RedSeg> red_segs;
-    std::vector<FpPSeg> fp_psegs;
+    std::vector<FprSeg> fpr_segs;
+    std::vector<const float*> parts;  // members' segment-sum scratch the plan was built on
     std::vector<BpPSeg> bp_psegs;
     int persistent = 0;  // tomo_batch_set_persistent mode (default: a launch per kernel variant)
     int* d_cursor = nullptr;
@@ -177,8 +181,12 @@ tomo_status build_plan(tomo_batch* b) {
     std::map<std::tuple<int, int, int, int, int>, std::vector<int4>> fpi;
     std::map<std::tuple<int, int, int, int, int>, size_t> fpsmem;
     std::map<std::tuple<int, int, int, int, int>, std::vector<int4>> bpi;
-    std::map<std::tuple<int, int, int, int, int>, std::vector<double>> fpcost, bpcost;  // per item, persistent
-    std::map<std::tuple<int, int, int, int, int>, std::vector<int>> fpclass;  // kernel body of a persistent item
+    std::map<std::tuple<int, int, int, int, int>, std::vector<double>> bpcost;  // per item, persistent
+    // row-vector form by (s, piece, chunk depth; 0 for the closing pass; -1: persistent; bytes of a voxel)
+    std::map<std::tuple<int, int, int, int>, std::vector<int4>> fpri;
+    std::map<std::tuple<int, int, int, int>, std::vector<double>> fprcost;
+    std::map<std::tuple<int, int, int, int>, size_t> fprsmem;
+    b->parts.clear();
     std::map<int, std::vector<ErrReduce>> reds;
     std::map<int, std::vector<VolJob>> vjobs;
     b->max_nsub = 0;
@@ -196,15 +204,19 @@ tomo_status build_plan(tomo_batch* b) {
         const int nsub = (N + upd - 1) / upd;
         b->max_nsub = std::max(b->max_nsub, nsub);
         b->has_fista = b->has_fista || p->fista;
+        // (a member's scratch may grow while its updates are planned: sized first)
+        for (int T : {upd, N - (nsub - 1) * upd}) {
+            FprPlan plan{};
+            handle_fpr_prepare(p, T, &plan);
+        }
+        b->parts.push_back(p->d_fppart);
         // rows the forward projector never writes must read as zero residual
         BCK(cudaMemsetAsync(p->d_errpart, 0, sizeof(double) * (size_t)N * g.h, b->stream));
         const int qp = fp_qp(g.w), nt = fp_threads(g.w);
         const int zc = fp_choose_zc(g.W, 1, p->vtype, nt);
         const int pk = p->vtype != kVolF32 ? 1 : 0;
         const int use_tma = fp_use_tma(g.W, p->vtype, p->vol());
-        int lq = 0;
-        while ((1 << lq) < qp) lq++;
-        const bool fp_persist = (b->persistent & kPersistFp) && fp_persist_supported(nt, zc);
+        const bool fp_persist = (b->persistent & kPersistFp) != 0;
         const int offset = (g.h > g.H && g.scale == 1) ? (g.h - g.H) / 2 : 0;
         const int j0 = std::max(0, (int)std::floor(offset * g.scale + 0.5));
         for (int s = 0; s < nsub; s++) {
@@ -234,23 +246,53 @@ tomo_status build_plan(tomo_batch* b) {
             a.h = g.h;
             a.row_off = g.fp_row_off;
             a.status = p->d_status;
-            const int di = (int)fp.size();
-            fp.push_back(a);
-            // persistent launches group by block size and chunk depth only (qp = pk = -1)
-            const auto key = fp_persist ? std::make_tuple(s, -1, nt, zc, -1) : std::make_tuple(s, qp, nt, zc, pk);
-            fpsmem[key] = std::max(fpsmem[key], fp_smem_bytes(zc, g.W, qp, 1, p->vtype));
-            auto& items = fpi[key];
-            // a row's tilt groups one after another: the staged planes are read again from L2
-            const int flags = use_tma | (fp_persist ? (lq << 1) | (pk << 4) : 0);
-            const double cost = (double)g.D * g.w * a.tilts_per_cta;  // ray-steps of a full item
-            for (int j = j0; j < g.h; j++)
-                for (int g0 = 0; g0 < T; g0 += a.tilts_per_cta) {
-                    items.push_back(make_int4(di, g0, j, flags));
-                    if (fp_persist) {
-                        fpcost[key].push_back(cost);
-                        fpclass[key].push_back(lq * 2 + pk);
-                    }
+            FprPlan plan{};
+            const int tc = handle_fpr_prepare(p, T, &plan);
+            if (tc > 0) {
+                for (int t0 = 0, c = 0; t0 < T; t0 += tc, c++) {
+                    FpLaunch q = a;
+                    q.T = std::min(tc, T - t0);
+                    q.tilts = a.tilts + t0;
+                    q.proj = a.proj + (size_t)t0 * p->npix;
+                    q.norm = a.norm + (size_t)t0 * p->npix;
+                    q.diff = a.diff + (size_t)t0 * p->npix;
+                    q.errpart = a.errpart + (size_t)t0 * g.h;
+                    q.rv = plan;
+                    q.rv.bulk = use_tma;
+                    q.tilts_per_cta = plan.tg;
+                    q.part = p->d_fppart;
+                    fpr_split_factor(&q);
+                    const int nrg = fpr_row_groups(q, &q.rv.jfirst);
+                    const int di = (int)fp.size();
+                    fp.push_back(q);
+                    const auto key = std::make_tuple(s, c, fp_persist ? -1 : plan.zc, fp_persist ? 0 : (int)vol_elem_bytes(p->vtype));
+                    fprsmem[key] = std::max(fprsmem[key], fpr_smem_bytes(plan));
+                    auto& items = fpri[key];
+                    // the tilt groups of a (window, row group, segment) one after another: its
+                    // columns come from L2 for all but the first
+                    for (int sg = 0; sg < plan.nseg; sg++)
+                        for (int rg = 0; rg < nrg; rg++)
+                            for (int win = 0; win < plan.nwin; win++)
+                                for (int g0 = 0; g0 < q.T; g0 += plan.tg) {
+                                    items.push_back(make_int4(di, g0 | (win << 16), q.rv.jfirst + 8 * rg, sg));
+                                    if (fp_persist)
+                                        fprcost[key].push_back((double)plan.seg * std::min(plan.tg, q.T - g0) * g.w /
+                                                               plan.nwin);
+                                }
+                    auto& fin = fpri[std::make_tuple(s, c, 0, 0)];
+                    for (int t = 0; t < q.T; t++)
+                        for (int j = j0; j < g.h; j++) fin.push_back(make_int4(di, t, j, 0));
                 }
+            } else {
+                const int di = (int)fp.size();
+                fp.push_back(a);
+                const auto key = std::make_tuple(s, qp, nt, zc, pk);
+                fpsmem[key] = std::max(fpsmem[key], fp_smem_bytes(zc, g.W, qp, 1, p->vtype));
+                // a row's tilt groups one after another: the staged planes are read again from L2
+                auto& items = fpi[key];
+                for (int j = j0; j < g.h; j++)
+                    for (int g0 = 0; g0 < T; g0 += a.tilts_per_cta) items.push_back(make_int4(di, g0, j, use_tma));
+            }
             reds[s].push_back(ErrReduce{a.errpart, p->d_err + slot, T, g.h});
             if (p->vtype != kVolF32)
                 vjobs[s].push_back(VolJob{p->vol(), p->d_vscale, p->d_vmax, p->vtype, g.W, g.H, g.D, p->d_status});
@@ -299,13 +341,10 @@ tomo_status build_plan(tomo_batch* b) {
     }
     // flatten; the lists of persistent launches go longest item first (stable, so a row's
     // tilt groups stay together)
-    // by kernel body first (CTAs that run the same body side by side share the instruction
-    // cache), then longest first
-    auto by_cost = [](std::vector<int4>& items, const std::vector<double>& cost, const std::vector<int>* cls) {
+    auto by_cost = [](std::vector<int4>& items, const std::vector<double>& cost) {
         std::vector<size_t> idx(items.size());
         for (size_t i = 0; i < idx.size(); i++) idx[i] = i;
         std::stable_sort(idx.begin(), idx.end(), [&](size_t x, size_t y) {
-            if (cls && (*cls)[x] != (*cls)[y]) return (*cls)[x] < (*cls)[y];
             return cost[x] > cost[y];
         });
         std::vector<int4> out(items.size());
@@ -317,28 +356,28 @@ tomo_status build_plan(tomo_batch* b) {
     b->fp_segs.clear();
     b->bp_segs.clear();
     b->red_segs.clear();
-    b->fp_psegs.clear();
+    b->fpr_segs.clear();
     b->bp_psegs.clear();
     b->n_cursor = 0;
     for (auto& kv : fpi) {
         const int s = std::get<0>(kv.first), nt = std::get<2>(kv.first), zc = std::get<3>(kv.first);
-        if (std::get<1>(kv.first) < 0) {
-            if (!(b->persistent & kPersistListOrder)) by_cost(kv.second, fpcost[kv.first], &fpclass[kv.first]);
-            const int n = (int)kv.second.size();
-            const int grid = std::min(n, fp_ctas_per_sm(nt) * sms);
-            b->fp_psegs.push_back(tomo_batch::FpPSeg{s, nt, zc, fpsmem[kv.first], (int)fp_all.size(), n,
-                                                     b->n_cursor++, grid});
-        } else {
-            b->fp_segs.push_back(tomo_batch::FpSeg{s, std::get<1>(kv.first), nt, zc, std::get<4>(kv.first),
-                                                   fpsmem[kv.first], (int)fp_all.size(), (int)kv.second.size()});
-        }
+        b->fp_segs.push_back(tomo_batch::FpSeg{s, std::get<1>(kv.first), nt, zc, std::get<4>(kv.first),
+                                               fpsmem[kv.first], (int)fp_all.size(), (int)kv.second.size()});
+        fp_all.insert(fp_all.end(), kv.second.begin(), kv.second.end());
+    }
+    for (auto& kv : fpri) {
+        const int zc = std::get<2>(kv.first);
+        if (zc < 0 && !(b->persistent & kPersistListOrder)) by_cost(kv.second, fprcost[kv.first]);
+        b->fpr_segs.push_back(tomo_batch::FprSeg{std::get<0>(kv.first), std::get<1>(kv.first), zc, std::get<3>(kv.first),
+                                                 zc ? fprsmem[kv.first] : 0, (int)fp_all.size(),
+                                                 (int)kv.second.size(), zc < 0 ? b->n_cursor++ : -1});
         fp_all.insert(fp_all.end(), kv.second.begin(), kv.second.end());
     }
     for (auto& kv : bpi) {
         const int s = std::get<0>(kv.first), vt = std::get<3>(kv.first);
         const bool san = std::get<1>(kv.first) != 0, pos = std::get<2>(kv.first) != 0, pairs = std::get<4>(kv.first) != 0;
         if (b->persistent & kPersistBp) {
-            if (!(b->persistent & kPersistListOrder)) by_cost(kv.second, bpcost[kv.first], nullptr);
+            if (!(b->persistent & kPersistListOrder)) by_cost(kv.second, bpcost[kv.first]);
             const int n = (int)kv.second.size();
             const int grid = std::min(n, bp_persist_ctas_per_sm(vt, pairs) * sms);
             b->bp_psegs.push_back(tomo_batch::BpPSeg{s, san, pos, vt, pairs, (int)bp_all.size(), n, b->n_cursor++,
@@ -423,14 +462,20 @@ tomo_status launch_step(tomo_batch* b) {
     for (tomo_projector* p : b->members) BCKS(handle_start_iteration(p));
     if (b->n_cursor > 0) BCK(cudaMemsetAsync(b->d_cursor, 0, sizeof(int) * b->n_cursor, b->stream));
     for (int s = 0; s < b->max_nsub; s++) {
-        std::vector<std::function<cudaError_t(cudaStream_t)>> jobs;
-        for (auto& sg : b->fp_psegs)
-            if (sg.s == s)
-                jobs.push_back([b, sg](cudaStream_t q) {
-                    return launch_fp_persist(sg.nt, sg.zc, b->d_fp, b->d_fp_items + sg.off, sg.n,
-                                             b->d_cursor + sg.cursor, sg.grid, sg.smem, q);
-                });
-        BCKS(run_side_by_side(b, jobs));
+        int pieces = 0;
+        for (auto& sg : b->fpr_segs)
+            if (sg.s == s) pieces = std::max(pieces, sg.c + 1);
+        for (int c = 0; c < pieces; c++) {
+            for (auto& sg : b->fpr_segs)
+                if (sg.s == s && sg.c == c && sg.zc > 0)
+                    BCK(launch_fpr_batch(sg.zc, sg.eb, b->d_fp, b->d_fp_items + sg.off, sg.n, sg.smem, b->stream));
+                else if (sg.s == s && sg.c == c && sg.zc < 0)
+                    BCK(launch_fpr_persist(b->d_fp, b->d_fp_items + sg.off, sg.n, b->d_cursor + sg.cursor,
+                                           std::min(sg.n, device_sms()), sg.smem, b->stream));
+            for (auto& sg : b->fpr_segs)
+                if (sg.s == s && sg.c == c && sg.zc == 0)
+                    BCK(launch_fp_finish_batch(b->d_fp, b->d_fp_items + sg.off, sg.n, b->stream));
+        }
         for (auto& sg : b->fp_segs)
             if (sg.s == s)
                 BCK(launch_fp_batch(sg.qp, sg.nt, b->d_fp, b->d_fp_items + sg.off, sg.n, sg.zc, sg.smem, sg.pk, b->stream));
@@ -566,6 +611,8 @@ tomo_status tomo_batch_iteration(tomo_batch* b, const double* relax, const int32
         upd[m] = update[m] == 0 ? N : std::min(update[m], N);
         fac[m] = (double)(float)(relax[m] / upd[m]);  // float factorimg (TomoReconstruction2.java:646)
     }
+    // a member's own calls may have moved its segment-sum scratch
+    for (size_t m = 0; b->plan_valid && m < M; m++) b->plan_valid = b->parts[m] == b->members[m]->d_fppart;
     if (!b->plan_valid || upd != b->upd || fac != b->factor) {
         b->upd = upd;
         b->factor = fac;

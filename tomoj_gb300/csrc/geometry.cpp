@@ -141,6 +141,8 @@ void build_fp_tables(const Geometry& g, const double* R, FpTilt* tilt, FpRay* ra
     const double bXmax = (double)((float)g.W + 1e-10f);
     tilt->step = to_fix(dirX);
     tilt->ninc = ninc;
+    tilt->ninc_hi = (float)ninc;
+    tilt->ninc_lo = (float)(ninc - (double)tilt->ninc_hi);
     const int D = g.D;
     // norm_sum is a float accumulating a double increment: norm(k) for k increments.
     std::vector<float> own;

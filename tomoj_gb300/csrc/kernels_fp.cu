@@ -1,9 +1,26 @@
 // Forward-projection dispatch: picks the kernel instantiation for the number of
 // detector columns each thread owns (QP = ceil(w / threads)); the kernel itself is in
 // fp_kernel.cuh and is compiled once per (threads, QP) pair (fp_kernel_q*.cu).
+#include <algorithm>
+#include <cmath>
+#include <functional>
+#include <queue>
+#include <vector>
+
+#include "device_util.cuh"
 #include "tomo_internal.h"
 
 namespace tomo {
+
+cudaError_t fpr_attr_z4();
+cudaError_t fpr_attr_z6();
+cudaError_t fpr_attr_z8();
+cudaError_t fpr_launch_z4(const FpLaunch& a, dim3 grid, size_t smem, cudaStream_t s);
+cudaError_t fpr_launch_z6(const FpLaunch& a, dim3 grid, size_t smem, cudaStream_t s);
+cudaError_t fpr_launch_z8(const FpLaunch& a, dim3 grid, size_t smem, cudaStream_t s);
+cudaError_t fpr_batch_z4(int eb, const FpLaunch* d, const int4* it, int n, size_t smem, cudaStream_t s);
+cudaError_t fpr_batch_z6(int eb, const FpLaunch* d, const int4* it, int n, size_t smem, cudaStream_t s);
+cudaError_t fpr_batch_z8(int eb, const FpLaunch* d, const int4* it, int n, size_t smem, cudaStream_t s);
 
 cudaError_t fp_launch_t256_q1(const FpLaunch& a, cudaStream_t s);
 cudaError_t fp_launch_t256_q2(const FpLaunch& a, cudaStream_t s);
@@ -20,12 +37,7 @@ cudaError_t fp_batch_t256_q2(const FpLaunch* d, const int4* it, int n, int zc, s
 cudaError_t fp_batch_t512_q2(const FpLaunch* d, const int4* it, int n, int zc, size_t smem, int pk, cudaStream_t s);
 cudaError_t fp_batch_t512_q4(const FpLaunch* d, const int4* it, int n, int zc, size_t smem, int pk, cudaStream_t s);
 cudaError_t fp_batch_t512_q8(const FpLaunch* d, const int4* it, int n, int zc, size_t smem, int pk, cudaStream_t s);
-cudaError_t fp_persist_attr_t256();
-cudaError_t fp_persist_attr_t512();
-cudaError_t fp_persist_t256(int zc, const FpLaunch* descs, const int4* items, int n_items, int* cursor, int grid,
-                            size_t smem, cudaStream_t s);
-cudaError_t fp_persist_t512(int zc, const FpLaunch* descs, const int4* items, int n_items, int* cursor, int grid,
-                            size_t smem, cudaStream_t s);
+cudaError_t fpr_persist_attr();
 
 // Raises the dynamic shared-memory limit of every forward-projector variant once,
 // outside any stream capture.
@@ -35,22 +47,11 @@ cudaError_t fp_init_attributes() {
     if ((e = fp_attr_t256_q2()) != cudaSuccess) return e;
     if ((e = fp_attr_t512_q2()) != cudaSuccess) return e;
     if ((e = fp_attr_t512_q4()) != cudaSuccess) return e;
-    if ((e = fp_persist_attr_t256()) != cudaSuccess) return e;
-    if ((e = fp_persist_attr_t512()) != cudaSuccess) return e;
+    if ((e = fpr_attr_z4()) != cudaSuccess) return e;
+    if ((e = fpr_attr_z6()) != cudaSuccess) return e;
+    if ((e = fpr_attr_z8()) != cudaSuccess) return e;
+    if ((e = fpr_persist_attr()) != cudaSuccess) return e;
     return fp_attr_t512_q8();
-}
-
-bool fp_persist_supported(int nt, int zc) { return (nt == 256 && zc == 16) || (nt == 512 && (zc == 16 || zc == 8)); }
-
-cudaError_t launch_fp_persist(int nt, int zc, const FpLaunch* descs, const int4* items, int n_items, int* cursor,
-                              int grid, size_t smem, cudaStream_t s) {
-    if (n_items <= 0) return cudaSuccess;
-    if (!fp_persist_supported(nt, zc) || smem > fp_smem_budget(nt) || grid <= 0) return cudaErrorInvalidValue;
-    const cudaError_t e = nt == 256 ? fp_persist_t256(zc, descs, items, n_items, cursor, grid, smem, s)
-                                    : fp_persist_t512(zc, descs, items, n_items, cursor, grid, smem, s);
-    if (e != cudaSuccess) return e;
-    count_launch();
-    return cudaGetLastError();
 }
 
 int fp_threads(int w) { return w <= 512 ? 256 : 512; }
@@ -136,6 +137,284 @@ cudaError_t launch_fp_separable(const FpLaunch& a, cudaStream_t s) {
         case 8: return fp_launch_t512_q8(a, s);
     }
     return cudaErrorInvalidValue;
+}
+
+// --- row-vector form ------------------------------------------------------------------------
+
+namespace {
+
+constexpr int kFinishThreads = 128;
+
+// a * b in FP32 for a double b = hi + lo (lo below half an ulp of hi): the product rounded
+// once from 48 bits (and its low part), without an FP64 operation per ray (this part's FP64
+// rate is 1/64 of FP32: two conversions and a product per ray would take longer than the
+// pass's memory traffic).
+struct F2 {
+    float hi, lo;
+};
+__device__ __forceinline__ F2 mul_split(float a, F2 b) {
+    const float p = a * b.hi;
+    const float e = fmaf(a, b.lo, fmaf(a, b.hi, -p));
+    const float r = p + e;
+    // an infinite or overflowing product keeps p (the correction is NaN)
+    return isfinite(p) ? F2{r, e - (r - p)} : F2{p, 0.0f};
+}
+
+// Running sum with its error (two-sum): hi + lo carries about 48 bits.
+__device__ __forceinline__ void add2(F2& s, float p, float pe) {
+    const float t = s.hi + p, u = t - s.hi;
+    s.lo += ((s.hi - (t - u)) + (p - u)) + pe;
+    s.hi = t;
+}
+
+// Projection, norm, difference and residual of one projection row from its segment sums
+// (the epilogue of fp_body with the sums read back, in segment order).  The squared
+// differences are summed in FP32 pairs with error terms, a warp's sums in FP64.  Bound by its
+// memory traffic (segment sums, ray table, measured row in; projection, norm and difference
+// out): 11 us for 7 tilts of 512 x 256 in 5 segments, where a form with seven FP64 operations
+// per ray took 27 us.
+__device__ __forceinline__ void finish_row(const FpLaunch& a, int b, int j) {
+    __shared__ double red[kFinishThreads / 32];
+    const int tilt = a.tilts[b];
+    const int r = a.two_rows ? a.rowmap[j] : j - a.row_off;
+    const bool row_in = r >= 0 && r < a.H;
+    // reduced storage: ray sums are in units of the row's slab scale (a power of two)
+    const float vsc = (a.vscale != nullptr && row_in) ? a.vscale[r] : 1.0f;
+    const F2 ninc{a.ftilt[tilt].ninc_hi, a.ftilt[tilt].ninc_lo}, fac{a.factor_hi, a.factor_lo};
+    const size_t seg_stride = (size_t)a.T * a.h * a.w, row = ((size_t)b * a.h + j) * a.w;
+    const float inv_seg = 1.0f / (float)a.rv.seg;
+    F2 e2{0.0f, 0.0f};
+    double far = 0.0;  // squares outside FP32's comfortable range
+    for (int i = threadIdx.x; i < a.w; i += kFinishThreads) {
+        const FpRay ray = a.rays[(size_t)tilt * a.w + i];
+        const float e = a.meas != nullptr ? a.meas[((size_t)tilt * a.h + j) * a.w + i] : 0.0f;
+        const int za = ray.zab & 0xFFFF, cnt = (int)((uint32_t)ray.zab >> 16);
+        const size_t o = row + i;
+        float th = __int_as_float(0x7fc00000), nrm = 0.0f;
+        if (cnt != 0 && row_in) {
+            // floor(z / seg): z + 1/2 keeps the product clear of whole numbers (z < 2^16)
+            const int s0 = (int)((za + 0.5f) * inv_seg), s1 = (int)((za + cnt - 0.5f) * inv_seg);
+            float sum = 0.0f;
+            for (int s = s0; s <= s1; s += 4) {
+                float v[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) v[q] = s + q <= s1 ? __ldcg(a.part + (s + q) * seg_stride + o) : 0.0f;
+#pragma unroll
+                for (int q = 0; q < 4; q++) sum += v[q];
+            }
+            th = mul_split(sum * vsc, ninc).hi;
+            nrm = ray.norm;
+        }
+        a.proj[o] = th;
+        a.norm[o] = nrm;
+        if (a.meas != nullptr) {
+            float d = 0.0f;
+            if (!isnan(e) && !isnan(th)) {
+                const F2 v = mul_split(__fdiv_rn(__fsub_rn(e, th), nrm), fac);
+                d = v.hi;
+                const float m = fabsf(d);
+                if ((m > 1e15f || m < 1e-15f) && d != 0.0f) {
+                    far += (double)d * d;
+                } else {
+                    const float p = d * d;
+                    add2(e2, p, fmaf(d, d, -p) + 2.0f * d * v.lo);
+                }
+            }
+            a.diff[o] = d;
+        }
+    }
+    if (a.meas != nullptr) {
+        // the lanes' sums in fixed order, without FP64 (an infinite sum has no error term)
+#pragma unroll
+        for (int q = 16; q > 0; q >>= 1) {
+            const float oh = __shfl_down_sync(0xffffffffu, e2.hi, q), ol = __shfl_down_sync(0xffffffffu, e2.lo, q);
+            add2(e2, oh, ol);
+        }
+        if (__any_sync(0xffffffffu, far != 0.0)) far = warp_sum(far);
+        if ((threadIdx.x & 31) == 0)
+            red[threadIdx.x >> 5] = (isfinite(e2.hi) ? (double)e2.hi + (double)e2.lo : (double)e2.hi) + far;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double sum = 0.0;
+            for (int k = 0; k < kFinishThreads / 32; k++) sum += red[k];
+            a.errpart[(size_t)b * a.h + j] = sum;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kFinishThreads) fp_finish_kernel(const __grid_constant__ FpLaunch a) {
+    finish_row(a, blockIdx.y, a.j0 + blockIdx.x);
+}
+
+// Batched form: block b runs items[b] = {problem, tilt, row, -}.
+__global__ void __launch_bounds__(kFinishThreads)
+    fp_finish_batch_kernel(const FpLaunch* __restrict__ descs, const int4* __restrict__ items) {
+    const int4 it = items[blockIdx.x];
+    finish_row(descs[it.x], it.y, it.z);
+}
+
+}  // namespace
+
+size_t fpr_smem_bytes(const FprPlan& p) { return kFprFixedSmem + (size_t)p.zc * p.pitch * (64 + 4 * p.rawrows); }
+
+// Time of a grid on `sms` SMs in units of a full segment's CTA: CTAs start in segment order,
+// `per_seg` each.  A segment away from the middle plane has fewer rays inside, the last one
+// fewer planes.
+static double grid_time(int nseg, int per_seg, double last, double lean, int sms) {
+    const double n = (double)nseg * per_seg;
+    auto weight = [&](int s) {
+        const double d = nseg > 1 ? std::fabs((s + 0.5) / nseg - 0.5) * 2 : 0.0;
+        return (s == nseg - 1 ? last : 1.0) * (1.0 - lean * d);
+    };
+    if (n > 4.0 * sms) {
+        double sum = 0;
+        for (int s = 0; s < nseg; s++) sum += weight(s);
+        return sum * per_seg / sms + 0.5;
+    }
+    std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
+    for (int k = 0; k < sms; k++) free_at.push(0.0);
+    double end = 0;
+    for (int s = 0; s < nseg; s++)
+        for (int k = 0; k < per_seg; k++) {
+            const double t = free_at.top() + weight(s);
+            free_at.pop();
+            free_at.push(t);
+            end = std::max(end, t);
+        }
+    return end;
+}
+
+// Cuts a projection into CTAs by a cost model (cycles of one SM): a plane costs half a cycle
+// per staged column (8 voxels transposed at 16 a cycle) and 18.4 cycles per ray block (256
+// samples at 13.9 a cycle), with one plane's worth of bookkeeping per chunk; a CTA costs
+// 12000 cycles besides (lists, first chunk, sums).  Fitted on 512 x 256 x 512: 7 tilts in 4 /
+// 5 / 8 / 13 / 16 segments 202 / 177 / 200 / 191 / 206 us, 41 tilts in 3 / 6 / 13 segments
+// 995 / 1022 / 1090 us; 256 x 64 x 256, 61 tilts in 4 / 7 / 8 segments 118 / 116 / 128 us;
+// 1024 x 256 x 256, 61 tilts in 6 windows of 3 segments 1567 us, 5 of 3 1655 us.
+// Deeper chunks leave narrower windows (the buffers hold zc * pitch columns), longer segments
+// wider margins around a window (tilts fan out by max_step columns per plane).
+FprPlan fpr_plan(const FprGeom& g, int T, int sms) {
+    FprPlan best{};
+    if (T <= 0 || g.w > 4096 || !(g.max_step <= 16.0) || !(g.max_space <= 64.0) || !(g.min_space > 0)) return best;
+    const int NB = (g.w + kFprRays - 1) / kFprRays, cap = kFprSlots * 16;
+    // eight projection rows touch the rows between their floors and one more
+    const int rawrows = g.row_step > 0 ? (int)std::ceil(7 * g.row_step) + 2 : 8;
+    if (rawrows > 16) return best;
+    const int nrg = (g.rows + 14) / 8;
+    double best_cost = 0;
+    for (int zc : {8, 6, 4}) {
+        const int room = (int)((kFprSmemMax - kFprFixedSmem) / ((size_t)zc * (64 + 4 * rawrows)));
+        for (int nch = 1; nch <= kFprMaxChunks; nch = nch < 8 ? nch + 1 : nch + (nch + 3) / 4) {
+            const int seg = std::min(nch, (g.D + zc - 1) / zc) * zc;
+            FprPlan p{};
+            p.zc = zc;
+            p.rawrows = rawrows;
+            p.seg = seg;
+            p.nseg = (g.D + seg - 1) / seg;
+            double cols;
+            int nbw;
+            double nba;
+            // pitches are multiples of 8: a staged row starts on a 16-byte boundary in 16 bits too
+            if (((g.W + 11) & ~7) <= room) {
+                p.nwin = 1;
+                p.xw = g.W;
+                p.pitch = (g.W + 11) & ~7;
+                cols = g.W + 4;
+                nbw = NB;
+                nba = NB;
+            } else {
+                // margins: the tilts' fan over half a segment, a block's width, rounding
+                const int half = (seg + 1) / 2 + 1;
+                const int margin = 2 * (int)std::ceil(half * g.max_step + 1) + 2 * (int)std::ceil((kFprRays - 1) * g.max_space + 2) + 16;
+                p.xw = (room & ~7) - margin;
+                if (p.xw < 64) {
+                    if (seg >= g.D || nch > 1) break;
+                    continue;
+                }
+                p.nwin = (g.W + p.xw - 1) / p.xw;
+                p.xw = (g.W + p.nwin - 1) / p.nwin;
+                p.pitch = (p.xw + margin + 7) & ~7;
+                cols = std::min<double>(g.W + 3, p.xw + half * g.max_step + kFprRays * g.max_space);
+                nbw = std::min(NB, (int)(p.xw / (kFprRays * g.min_space)) + 2);
+                nba = std::min<double>(NB, p.xw / (kFprRays * std::min(1.2 * g.min_space, g.max_space)) + 0.5);
+            }
+            int tg = std::max(1, std::min({kFprMaxTilts, T, cap / nbw}));
+            const int ntg = (T + tg - 1) / tg;
+            tg = (T + ntg - 1) / ntg;
+            p.tg = tg;
+            const int passes = (nbw * tg + cap - 1) / cap;
+            // (whole rows of 16 blocks: every warp has as many ray blocks as the busiest)
+            double per_plane = passes * 0.5 * cols + 18.4 * 16.0 * std::ceil(tg * nba / 16.0) * (1.0 + 1.0 / zc);
+            per_plane = std::max(per_plane, 1200.0 / zc) + 600.0 / zc;
+            const double last = (double)(g.D - (p.nseg - 1) * seg) / seg;
+            const double lean = std::min(0.35, 0.2 * g.D * g.max_step / g.W);
+            const double cost = grid_time(p.nseg, ntg * p.nwin * nrg, last, lean, sms) *
+                                    (std::min(seg, g.D) * per_plane + 12000.0) +
+                                (double)p.nseg * T * g.h * g.w * 8.0 / 3400.0;
+            if (best.zc == 0 || cost < best_cost) {
+                best = p;
+                best_cost = cost;
+            }
+            if (seg >= g.D) break;
+        }
+    }
+    return best;
+}
+
+int fpr_row_groups(const FpLaunch& a, int* jfirst) {
+    if (a.two_rows) {
+        *jfirst = a.j0;
+        return (a.j1 - a.j0 + 7) / 8;
+    }
+    // groups end at the volume's last row, whose samples take another form
+    const int lo = std::max(a.j0, a.row_off), hi = std::min(a.j1, a.row_off + a.H);
+    if (hi <= lo) return 0;
+    const int end = a.row_off + a.H;
+    const int first = end - (end - lo + 7) / 8 * 8;
+    *jfirst = first;
+    return (hi - first + 7) / 8;
+}
+
+void fpr_split_factor(FpLaunch* a) {
+    a->factor_hi = (float)a->factor;
+    a->factor_lo = std::isfinite(a->factor_hi) ? (float)(a->factor - (double)a->factor_hi) : 0.0f;
+}
+
+cudaError_t launch_fpr(const FpLaunch& a0, cudaStream_t s) {
+    FpLaunch a = a0;
+    if (a.T <= 0 || a.j1 <= a.j0) return cudaSuccess;
+    const int nrg = fpr_row_groups(a, &a.rv.jfirst);
+    a.tilts_per_cta = a.rv.tg;
+    fpr_split_factor(&a);
+    a.rv.bulk = fp_use_tma(a.W, a.vtype, a.vol);
+    if (nrg > 0) {
+        const dim3 grid((unsigned)((a.T + a.rv.tg - 1) / a.rv.tg * a.rv.nwin), (unsigned)nrg, (unsigned)a.rv.nseg);
+        const size_t sm = fpr_smem_bytes(a.rv);
+        const cudaError_t e = a.rv.zc == 8   ? fpr_launch_z8(a, grid, sm, s)
+                              : a.rv.zc == 6 ? fpr_launch_z6(a, grid, sm, s)
+                                             : fpr_launch_z4(a, grid, sm, s);
+        if (e != cudaSuccess) return e;
+        count_launch();
+    }
+    fp_finish_kernel<<<dim3((unsigned)(a.j1 - a.j0), (unsigned)a.T), kFinishThreads, 0, s>>>(a);
+    count_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t launch_fpr_batch(int zc, int eb, const FpLaunch* descs, const int4* items, int n, size_t smem,
+                             cudaStream_t s) {
+    if (n <= 0) return cudaSuccess;
+    count_launch();
+    return zc == 8   ? fpr_batch_z8(eb, descs, items, n, smem, s)
+           : zc == 6 ? fpr_batch_z6(eb, descs, items, n, smem, s)
+                     : fpr_batch_z4(eb, descs, items, n, smem, s);
+}
+
+cudaError_t launch_fp_finish_batch(const FpLaunch* descs, const int4* items, int n, cudaStream_t s) {
+    if (n <= 0) return cudaSuccess;
+    fp_finish_batch_kernel<<<n, kFinishThreads, 0, s>>>(descs, items);
+    count_launch();
+    return cudaGetLastError();
 }
 
 }  // namespace tomo

@@ -234,6 +234,42 @@ int fp_split(tomo_projector* p, int T, int rows, int tpc) {
     return P;
 }
 
+// Row-vector form: its plan for T tilts and the tilts per launch (see handle_fpr_prepare).
+// The segment sums of a launch take at most eight times the series' size (the handle holds
+// six such buffers) and 1 GiB; more tilts run in further launches.  Volumes that hold NaN or Inf stay
+// on the one-row form, whose samples treat them as before.
+int fpr_prepare(tomo_projector* p, int T, FprPlan* plan) {
+    const Geometry& g = p->g;
+    if (T <= 0 || !g.separable || p->vol_flag()) return 0;
+    FprGeom fg{g.W, g.H, g.D, g.w, g.h, p->vtype, p->fp_max_step, p->fp_max_space, p->fp_min_space,
+               g.fractional ? g.h : g.H, g.fractional ? 1.0 / g.scale : 0.0};
+    const FprPlan* have = nullptr;
+    for (auto& q : p->fpr_plans)
+        if (q.first == T) have = &q.second;
+    if (!have) {
+        if (p->fpr_plans.size() >= 16) p->fpr_plans.clear();
+        p->fpr_plans.emplace_back(T, fpr_plan(fg, T, p->sms));
+        have = &p->fpr_plans.back().second;
+    }
+    *plan = *have;
+    if (plan->zc == 0) return 0;
+    const size_t per_tilt = (size_t)plan->nseg * p->npix;
+    const size_t lim = std::min<size_t>((size_t)8 * g.N * p->npix, (size_t)1 << 28);
+    int tc = (int)std::min<size_t>((size_t)T, std::max<size_t>(1, lim / per_tilt));
+    if (tc < T && tc >= plan->tg) tc -= tc % plan->tg;
+    if (p->tilts_per_cta > 0) plan->tg = std::min({p->tilts_per_cta, kFprMaxTilts, T});
+    const size_t need = per_tilt * (size_t)tc;
+    if (need > p->fppart_cap) {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(p->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return 0;
+        free_n(p, &p->d_fppart, p->fppart_cap);
+        p->fppart_cap = 0;
+        if (alloc_n(p, &p->d_fppart, need) != TOMO_OK) return 0;
+        p->fppart_cap = need;
+    }
+    return tc;
+}
+
 // Forward row map of the fractional-row form for projections whose tasks start at
 // row j0 (uploaded when j0 changes; the host copy stays alive for captured copies).
 tomo_status ensure_fp_rowmap(tomo_projector* p, int j0) {
@@ -245,6 +281,36 @@ tomo_status ensure_fp_rowmap(tomo_projector* p, int j0) {
     CK(cudaMemcpyAsync(p->d_fprow, p->h_fprow.data(), sizeof(int) * g.h, cudaMemcpyHostToDevice, p->stream));
     CK(cudaMemcpyAsync(p->d_fpyf, p->h_fpyf.data(), sizeof(float) * g.h, cudaMemcpyHostToDevice, p->stream));
     p->fprow_j0 = j0;
+    return TOMO_OK;
+}
+
+// Launches the separable projection `a` of a.T tilts: the row-vector form where it applies,
+// else the one-row form (depth-split on short grids unless `whole`: a row range of a
+// row-stream iteration).
+tomo_status launch_fp(tomo_projector* p, FpLaunch a, bool whole = false) {
+    FprPlan plan{};
+    const int tc = fpr_prepare(p, a.T, &plan);
+    if (tc > 0) {
+        const int T = a.T;
+        a.rv = plan;
+        a.part = p->d_fppart;
+        FpLaunch b = a;
+        for (int t0 = 0; t0 < T; t0 += tc) {
+            b.T = std::min(tc, T - t0);
+            b.tilts = a.tilts + t0;
+            b.proj = a.proj + (size_t)t0 * p->npix;
+            b.norm = a.norm + (size_t)t0 * p->npix;
+            b.diff = a.diff + (size_t)t0 * p->npix;
+            b.errpart = a.errpart + (size_t)t0 * a.h;
+            CK(launch_fpr(b, p->stream));
+        }
+        return TOMO_OK;
+    }
+    a.tilts_per_cta = auto_tilts_per_cta(p, a.T, a.j1 - a.j0);
+    a.zparts = whole ? 1 : fp_split(p, a.T, a.j1 - a.j0, a.tilts_per_cta);
+    a.part = p->d_fppart;
+    a.tickets = p->d_tickets;
+    CK(launch_fp_separable(a, p->stream));
     return TOMO_OK;
 }
 
@@ -321,10 +387,6 @@ tomo_status run_fp(tomo_projector* p, const int* d_tilts, int T, int y0, bool wi
     a.factor = factor;
     a.j0 = j0;
     a.j1 = j1;
-    a.tilts_per_cta = auto_tilts_per_cta(p, T, j1 - j0);
-    a.zparts = fp_split(p, T, j1 - j0, a.tilts_per_cta);
-    a.part = p->d_fppart;
-    a.tickets = p->d_tickets;
     if (g.fractional) {
         CKS(ensure_fp_rowmap(p, j0));
         a.rowmap = p->d_fprow;
@@ -339,7 +401,7 @@ tomo_status run_fp(tomo_projector* p, const int* d_tilts, int T, int y0, bool wi
     a.row_off = g.fp_row_off;
     a.status = p->d_status;
     a.hold_first_copy = p->hold_first_copy;
-    CK(launch_fp_separable(a, p->stream));
+    CKS(launch_fp(p, a));
     if (p->params.long_object) {
         CK(launch_long_object(norm, T, g.h, g.w, p->stream));
         if (with_diff)
@@ -370,8 +432,6 @@ tomo_status run_fp_range(tomo_projector* p, const int* d_tilts, int T, int j0, i
     a.factor = factor;
     a.j0 = j0;
     a.j1 = j1;
-    a.tilts_per_cta = auto_tilts_per_cta(p, T, j1 - j0);
-    a.zparts = 1;
     a.W = g.W;
     a.H = g.H;
     a.D = g.D;
@@ -380,8 +440,7 @@ tomo_status run_fp_range(tomo_projector* p, const int* d_tilts, int T, int j0, i
     a.row_off = g.fp_row_off;
     a.status = p->d_status;
     a.hold_first_copy = p->hold_first_copy;
-    CK(launch_fp_separable(a, p->stream));
-    return TOMO_OK;
+    return launch_fp(p, a, true);
 }
 
 tomo_status apply_weighting(tomo_projector* p, float* imgs, int T) {
@@ -572,6 +631,7 @@ tomo_status handle_need_series(tomo_projector* p) { return need_series(p); }
 tomo_status handle_start_iteration(tomo_projector* p) { return start_iteration(p); }
 tomo_status handle_end_iteration(tomo_projector* p) { return end_iteration(p); }
 int handle_tilts_per_cta(const tomo_projector* p, int T) { return auto_tilts_per_cta(p, T, 0); }
+int handle_fpr_prepare(tomo_projector* p, int T, FprPlan* plan) { return fpr_prepare(p, T, plan); }
 }  // namespace tomo
 
 extern "C" {
@@ -819,6 +879,16 @@ static tomo_status setup_geometry(tomo_projector* p) {
             return fail(TOMO_ERR_UNSUPPORTED, "16-bit volume storage needs scale 1");
     }
     if (sep) {
+        p->fpr_plans.clear();
+        p->fp_max_step = p->fp_max_space = 0;
+        p->fp_min_space = 1e30;
+        for (int t = 0; t < N; t++) {
+            const double* R = &p->euler[9 * t];
+            const double space = 1.0 / std::fabs(R[0] * g.scale);
+            p->fp_max_step = std::max(p->fp_max_step, std::fabs(R[2] / R[0]));
+            p->fp_max_space = std::max(p->fp_max_space, space);
+            p->fp_min_space = std::min(p->fp_min_space, space);
+        }
         g.fp_row_off = (int)(g.pc[1] - g.vc[1]);
         g.bp_row_off = (int)(g.pc[3] - g.vc[1]);
         std::vector<FpTilt> ft(N);
@@ -1694,8 +1764,11 @@ tomo_status tomo_run_ossart(tomo_projector* p, int32_t n_iter, double relax, int
         // depth-split scratch for the subset sizes of this run, before any capture
         int j0, j1;
         fp_rows(p, y0, &j0, &j1);
-        for (int T : {upd, N - (nsub - 1) * upd})
-            if (T > 0) fp_split(p, T, j1 - j0, auto_tilts_per_cta(p, T, j1 - j0));
+        for (int T : {upd, N - (nsub - 1) * upd}) {
+            FprPlan plan{};
+            if (T > 0 && g.separable && fpr_prepare(p, T, &plan) == 0)
+                fp_split(p, T, j1 - j0, auto_tilts_per_cta(p, T, j1 - j0));
+        }
         if (g.separable && g.fractional) CKS(ensure_fp_rowmap(p, j0));
     }
     // row streams: integral separable FP32 geometry without long-object compensation

@@ -124,6 +124,9 @@ struct tomo_projector {
     cudaStream_t rs_reduce = nullptr;
     std::vector<cudaEvent_t> rs_ev;  // fork, per-(subset, range) forward-done, joins
     int sms = 0;            // multiprocessors of the device
+    // series geometry of the row-vector forward projector (fpr_plan)
+    double fp_max_step = 0, fp_max_space = 0, fp_min_space = 0;
+    std::vector<std::pair<int, tomo::FprPlan>> fpr_plans;  // by tilts per update, for this geometry
     // forward-projector depth split scratch (partial ray sums, per-group tickets)
     float* d_fppart = nullptr;
     size_t fppart_cap = 0;  // floats
@@ -147,4 +150,8 @@ tomo_status handle_need_series(tomo_projector* p);
 tomo_status handle_start_iteration(tomo_projector* p);
 tomo_status handle_end_iteration(tomo_projector* p);
 int handle_tilts_per_cta(const tomo_projector* p, int T);
+// Plan of the row-vector forward projector for updates of T tilts and the tilts one launch
+// takes (the partial sums' scratch is bounded); 0: the handle's projections run the one-row
+// form.  Allocates the scratch unless the handle's stream is being captured.
+int handle_fpr_prepare(tomo_projector* p, int T, tomo::FprPlan* plan);
 }  // namespace tomo

@@ -50,6 +50,7 @@ struct alignas(16) FpRay {
 struct alignas(16) FpTilt {
     long long step;  // fixed-point dirX
     double ninc;     // normIncrement
+    float ninc_hi, ninc_lo;  // ninc as a sum of two floats
 };
 
 // Backprojection of tilt t: xx(x, z) = K + x * C + z * S (fixed point, volume
@@ -114,6 +115,28 @@ enum VolType : int { kVolF32 = 0, kVolBF16 = 1, kVolF16 = 2 };
 #endif
 TOMO_HD inline size_t vol_elem_bytes(int vt) { return vt == kVolF32 ? 4 : 2; }
 
+// Row-vector forward projector (fpr_kernel.cuh): how a launch is cut into CTAs.
+constexpr int kFprMaxTilts = 16;               // tilts per CTA
+constexpr int kFprRays = 32;                   // rays per block
+#ifndef FPR_SLOTS
+#define FPR_SLOTS 7
+#endif
+constexpr int kFprSlots = FPR_SLOTS;                   // blocks per warp (16 warps)
+constexpr int kFprMaxChunks = 64;              // chunks per segment
+constexpr size_t kFprFixedSmem = 25088;        // shared memory besides the plane buffers
+constexpr size_t kFprSmemMax = 227 * 1024;
+struct FprPlan {
+    int zc;       // planes per chunk (4, 6 or 8; 0: not usable for this geometry)
+    int seg;      // planes per segment (a multiple of zc); segments are summed in order
+    int nseg;
+    int nwin, xw; // column windows and their width at a segment's middle plane
+    int pitch;    // columns of a plane buffer
+    int tg;       // tilts per CTA
+    int rawrows;  // volume rows staged per plane (8; fractional rows: the rows eight of them touch)
+    int bulk;     // rows start on 16-byte boundaries: the first chunk comes by bulk copies
+    int jfirst;   // projection row of the first row group
+};
+
 // Device kernels (launch wrappers in the .cu files).  All return cudaError_t of the launch.
 struct FpLaunch {
     const void* vol;        // [D][H][W] of vtype
@@ -129,6 +152,7 @@ struct FpLaunch {
     float* diff;            // [T][h][w] (written when meas != nullptr)
     double* errpart;        // [T][h] per-row sum of squared differences
     double factor;          // relaxation factor passed to projectAndDifference
+    float factor_hi, factor_lo;  // factor as a sum of two floats (row-vector form)
     int j0, j1;             // projection rows to compute
     int tilts_per_cta;
     int W, H, D, w, h;
@@ -150,9 +174,35 @@ struct FpLaunch {
     // are never issued, so its mbarrier wait runs out after kHoldWaitTries polls and the
     // CTA reports kStatusTimeout and returns (nothing is in flight).  0 in normal use.
     int hold_first_copy;
+    FprPlan rv;             // row-vector form (rv.zc != 0): part holds [nseg][T][h][w] segment sums
 };
 constexpr uint32_t kHoldWaitTries = 1u << 12;
 cudaError_t launch_fp_separable(const FpLaunch& a, cudaStream_t s);
+// Row-vector form: the plan for T tilts of a series, and its launch (projector, then the
+// pass that adds the segments and writes projections, norms and residuals).  The cut into
+// segments depends on the series' geometry and T only, so that every caller (single, row
+// range, batch) gets the same sums.
+struct FprGeom {
+    int W, H, D, w, h, vtype;
+    double max_step, max_space, min_space;  // |columns per plane|, |columns per ray| over the series
+    int rows;                               // projection rows with a volume row
+    double row_step;                        // volume rows per projection row (0: whole rows)
+};
+FprPlan fpr_plan(const FprGeom& g, int T, int sms);
+// Row groups of projection rows [j0, j1): sets rv.jfirst, returns their number.
+int fpr_row_groups(const FpLaunch& a, int* jfirst);
+cudaError_t launch_fpr(const FpLaunch& a, cudaStream_t s);
+size_t fpr_smem_bytes(const FprPlan& p);
+void fpr_split_factor(FpLaunch* a);  // factor_hi, factor_lo from factor
+// (eb: bytes of a stored voxel, the same for every descriptor of a launch.)
+cudaError_t launch_fpr_batch(int zc, int eb, const FpLaunch* descs, const int4* items, int n, size_t smem,
+                             cudaStream_t s);
+// Persistent form: `grid` resident CTAs take items in list order through the atomic *cursor
+// (zero before the launch), whatever their chunk depth.
+cudaError_t launch_fpr_persist(const FpLaunch* descs, const int4* items, int n_items, int* cursor, int grid,
+                               size_t smem, cudaStream_t s);
+// The closing pass of many problems: block b runs items[b] = {problem, tilt, row, -}.
+cudaError_t launch_fp_finish_batch(const FpLaunch* descs, const int4* items, int n, cudaStream_t s);
 // Any geometry (kernels_generic.cu): one thread per ray / voxel in the reference's
 // double arithmetic.  proj/norm are [T][h][w] in batch order.
 struct FpGenericLaunch {
@@ -277,13 +327,6 @@ size_t fp_smem_bytes(int ZC, int W, int qp, int rows = 1, int vtype = kVolF32);
 // pk = 1 when every descriptor of the launch has a 16-bit volume, 0 when all are FP32.
 cudaError_t launch_fp_batch(int qp, int nt, const FpLaunch* descs, const int4* items, int n_items, int zc,
                             size_t smem, int pk, cudaStream_t s);
-// Persistent batched forward projection: `grid` resident CTAs of nt threads take items
-// {descriptor, first tilt, row, flags} in list order through the atomic *cursor (zero
-// before the launch); flags: bit 0 bulk copies, bits 1-3 log2 QP, bit 4 16-bit pairs.
-// One kernel per (nt, zc) serves every QP of its block size and both pair kinds.
-bool fp_persist_supported(int nt, int zc);
-cudaError_t launch_fp_persist(int nt, int zc, const FpLaunch* descs, const int4* items, int n_items, int* cursor,
-                              int grid, size_t smem, cudaStream_t s);
 cudaError_t fp_init_attributes();
 cudaError_t misc_init_attributes();
 cudaError_t launch_reduce_err(const double* errpart, double* err, int T, int h, cudaStream_t s);
