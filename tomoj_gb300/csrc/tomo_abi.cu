@@ -1100,9 +1100,19 @@ static tomo_status volume_copy(tomo_projector* p, float* host_or_dev, int on_dev
         CK(cudaStreamSynchronize(p->stream));
         return TOMO_OK;
     }
-    // reduced storage: blocks of rows through the FP32 staging buffer
+    // reduced storage: a device buffer is packed or unpacked in one pass, straight from or into
+    // it; host buffers (and any the device cannot address itself) go through the FP32 staging
+    // buffer in blocks of rows
     size_t cap = 0;
-    CKS(ensure_vtmp(p, &cap));
+    cudaPointerAttributes at{};
+    const bool direct = on_device && cudaPointerGetAttributes(&at, host_or_dev) == cudaSuccess &&
+                        at.type == cudaMemoryTypeDevice && at.device == p->device;
+    if (direct) {
+        cap = rows;
+    } else {
+        cudaGetLastError();
+        CKS(ensure_vtmp(p, &cap));
+    }
     // a whole new volume: the old row maxima must not count towards its maximum
     if (to_dev && rows == (size_t)g.H) CK(cudaMemsetAsync(p->d_vmax, 0, sizeof(unsigned) * g.H, p->stream));
     kind = on_device ? cudaMemcpyDeviceToDevice : (to_dev ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost);
@@ -1110,17 +1120,20 @@ static tomo_status volume_copy(tomo_projector* p, float* host_or_dev, int on_dev
         const size_t n = std::min(cap, rows - a);
         float* user = host_or_dev + a * g.W;  // row a of the caller's [D][rows][W] buffer
         const int r0 = y0 + (int)a;
+        float* f32 = direct ? user : p->d_vtmp;  // [D][n][W]
         if (to_dev) {
-            CK(cudaMemcpy2DAsync(p->d_vtmp, sizeof(float) * g.W * n, user, sizeof(float) * g.W * rows,
-                                 sizeof(float) * g.W * n, g.D, kind, p->stream));
+            if (!direct)
+                CK(cudaMemcpy2DAsync(f32, sizeof(float) * g.W * n, user, sizeof(float) * g.W * rows,
+                                     sizeof(float) * g.W * n, g.D, kind, p->stream));
             CK(cudaMemsetAsync(p->d_vmax + r0, 0, sizeof(unsigned) * n, p->stream));
-            CK(launch_vol_rowmax(p->d_vtmp, (int)n, r0, g.W, g.H, g.D, p->d_vmax, p->stream));
-            CK(launch_vol_pack(p->d_vtmp, (int)n, r0, g.W, g.H, g.D, p->vtype, p->vol(), p->d_vscale, p->d_vmax, false,
+            CK(launch_vol_rowmax(f32, (int)n, r0, g.W, g.H, g.D, p->d_vmax, p->stream));
+            CK(launch_vol_pack(f32, (int)n, r0, g.W, g.H, g.D, p->vtype, p->vol(), p->d_vscale, p->d_vmax, false,
                                p->d_status, p->stream));
         } else {
-            CK(launch_vol_unpack(p->vol(), p->vtype, p->d_vscale, (int)n, r0, g.W, g.H, g.D, p->d_vtmp, p->stream));
-            CK(cudaMemcpy2DAsync(user, sizeof(float) * g.W * rows, p->d_vtmp, sizeof(float) * g.W * n,
-                                 sizeof(float) * g.W * n, g.D, kind, p->stream));
+            CK(launch_vol_unpack(p->vol(), p->vtype, p->d_vscale, (int)n, r0, g.W, g.H, g.D, f32, p->stream));
+            if (!direct)
+                CK(cudaMemcpy2DAsync(user, sizeof(float) * g.W * rows, f32, sizeof(float) * g.W * n,
+                                     sizeof(float) * g.W * n, g.D, kind, p->stream));
         }
         // the staging buffer is reused by the next block
         CK(cudaStreamSynchronize(p->stream));
