@@ -14,51 +14,131 @@ namespace {
 // inverse-map every output pixel through Tinv around (w/2, h/2), Java (int) truncation,
 // bilinear in double with the floor pixel on the last row/column, optional
 // (x - mean) / stdDev, and the TiltSeries fill policy outside the image.
-__global__ void align_kernel(const float* __restrict__ raw, float* __restrict__ out, const double* __restrict__ tinv,
-                             const double* __restrict__ stats, int w, int h, int normalize, int fill,
-                             const unsigned char* __restrict__ identity) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y;
-    const int t = blockIdx.z;
-    if (i >= w) return;
-    const float* un = raw + (size_t)t * w * h;
+
+// One pixel in the reference's double expressions (pix before normalisation; false: outside).
+__device__ __noinline__ bool align_pixel_exact(const float* __restrict__ un, const double* __restrict__ T, int i, int j,
+                                               int w, int h, float* pix) {
+    // T: {i00, i10, i01, i11, i02, i12}
+    const double cx = w / 2.0, cy = h / 2.0;
+    const double px = (double)i - cx, jc = (double)j - cy;
+    const double xx = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(T[0], px), __dmul_rn(T[2], jc)), T[4]), cx);
+    const double yy = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(T[1], px), __dmul_rn(T[3], jc)), T[5]), cy);
+    const int ix0 = __double2int_rz(xx), iy0 = __double2int_rz(yy);
+    const double dx0 = __dsub_rn(xx, (double)ix0), dy0 = __dsub_rn(yy, (double)iy0);
+    if (ix0 < 0 || ix0 >= w || iy0 < 0 || iy0 >= h) return false;
+    if (ix0 == w - 1 || iy0 == h - 1) {
+        *pix = un[ix0 + (size_t)iy0 * w];
+        return true;
+    }
+    const double fac4 = __dmul_rn(dx0, dy0);
+    const size_t pos = ix0 + (size_t)iy0 * w;
+    const double v1 = un[pos], v3 = un[pos + w], v2 = un[pos + 1], v4 = un[pos + 1 + w];
+    const double w1 = __dadd_rn(__dsub_rn(__dsub_rn(1.0, dx0), dy0), fac4);
+    const double acc = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(v1, w1), __dmul_rn(v2, __dsub_rn(dx0, fac4))),
+                                           __dmul_rn(v3, __dsub_rn(dy0, fac4))),
+                                 __dmul_rn(v4, fac4));
+    *pix = __double2float_rn(acc);
+    return true;
+}
+
+// Pairs of floats (hi + lo, about 48 bits): a + t (b - a) for float or pair a, b and pair t.
+struct FPair {
+    float hi, lo;
+};
+__device__ __forceinline__ FPair pair_sum(float a, float b) {
+    const float s = a + b, u = s - a;
+    return FPair{s, (a - (s - u)) + (b - u)};
+}
+__device__ __forceinline__ FPair pair_lerp(FPair a, FPair b, FPair t) {
+    FPair d = pair_sum(b.hi, -a.hi);
+    d.lo += b.lo - a.lo;
+    const float p = t.hi * d.hi;
+    const float e = fmaf(t.hi, d.hi, -p) + (t.hi * d.lo + t.lo * d.hi);
+    FPair r = pair_sum(a.hi, p);
+    r.lo += a.lo + e;
+    return r;
+}
+
+// One pixel from 64-bit fixed-point coordinates (2^-48 pixel) and bilinear weights and sums in
+// pairs of floats, rounded once at the end: what double arithmetic gives to a few parts in
+// 2^46.  0: outside, 1: *pix set, 2: not decided here (a coordinate within 2^-20 of a whole
+// pixel, where truncation is the reference's double rounding's, or neighbours that are not
+// finite, or so large or small that a pair would lose bits).
+__device__ __forceinline__ int align_pixel_fixed(const float* __restrict__ un, const long long* __restrict__ F, int md,
+                                                 int i, int j, int w, int h, float* pix) {
+    const long long X = F[0] * i + F[2] * j + F[4], Y = F[1] * i + F[3] * j + F[5];
+    constexpr long long kOne = 1LL << 48, kNear = 1LL << 28;
+    const long long nx = md & 4 ? 0 : kNear, ny = md & 8 ? 0 : kNear;
+    if (((X + nx) & (kOne - 1)) < 2 * nx || ((Y + ny) & (kOne - 1)) < 2 * ny) return 2;
+    // truncation toward zero: a coordinate in (-1, 0) takes pixel 0 with a negative fraction
+    const int ix = X >= 0 ? (int)(X >> 48) : -(int)(-X >> 48), iy = Y >= 0 ? (int)(Y >> 48) : -(int)(-Y >> 48);
+    if (ix < 0 || ix >= w || iy < 0 || iy >= h) return 0;
+    const size_t pos = ix + (size_t)iy * w;
+    const float v1 = un[pos];
+    if (ix == w - 1 || iy == h - 1) {
+        *pix = v1;
+        return 1;
+    }
+    const float v2 = un[pos + 1], v3 = un[pos + w], v4 = un[pos + 1 + w];
+    const float mag = fabsf(v1) + fabsf(v2) + fabsf(v3) + fabsf(v4);
+    if (!(mag < 1e38f) || (mag > 0.0f && mag < 1e-30f)) return 2;
+    auto frac = [](long long f) {  // |f| < 2^48: both parts are exact
+        return FPair{(float)(int)(f >> 24) * (1.0f / 16777216.0f),
+                     (float)(unsigned)(f & 0xFFFFFF) * (1.0f / 16777216.0f / 16777216.0f)};
+    };
+    const FPair dx = frac(X - ((long long)ix << 48)), dy = frac(Y - ((long long)iy << 48));
+    const FPair top = pair_lerp(FPair{v1, 0.0f}, FPair{v2, 0.0f}, dx);
+    const FPair bot = pair_lerp(FPair{v3, 0.0f}, FPair{v4, 0.0f}, dx);
+    const FPair r = pair_lerp(top, bot, dy);
+    *pix = r.hi + r.lo;
+    return 1;
+}
+
+// mode per image: 0 double expressions, 1 identity, 2 fixed-point coordinates (fix: {x, y per
+// column, x, y per row, x, y at pixel (0, 0)} times 2^48) with + 4 and + 8 where x and y are
+// exact in both forms (whole or dyadic shifts).  flags: bit 0 a NaN was written, bit 1 an
+// infinity.  This part's FP64 rate is 1/64 of FP32: 61 images of 512 x 256 took 628
+// us in doubles and take 65 us in fixed point and float pairs, with the scan for
+// non-finite pixels (9 us) in the same pass.
+constexpr int kAlignPix = 4;  // pixels per thread
+
+__global__ void __launch_bounds__(256) align_kernel(const float* __restrict__ raw, float* __restrict__ out,
+                                                    const double* __restrict__ tinv, const long long* __restrict__ fix,
+                                                    const double* __restrict__ stats, int w, int h, int normalize,
+                                                    int fill, const unsigned char* __restrict__ mode, int* flags) {
+    const int t = blockIdx.y;
+    const size_t npix = (size_t)w * h;
+    const float* un = raw + t * npix;
+    float* dst = out + t * npix;
+    const int md = mode[t];
     const double mean = stats ? stats[2 * t] : 0.0;
     const double sd = stats ? stats[2 * t + 1] : 1.0;
-    float pix;
-    if (identity[t]) {
-        const float v = un[(size_t)j * w + i];
-        pix = normalize ? __double2float_rn(__ddiv_rn(__dsub_rn((double)v, mean), sd)) : v;
-    } else {
-        const double* T = tinv + 6 * t;  // {i00, i10, i01, i11, i02, i12}
-        const double cx = w / 2.0, cy = h / 2.0;
-        const double px = (double)i - cx, jc = (double)j - cy;
-        const double xx = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(T[0], px), __dmul_rn(T[2], jc)), T[4]), cx);
-        const double yy = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(T[1], px), __dmul_rn(T[3], jc)), T[5]), cy);
-        const int ix0 = __double2int_rz(xx), iy0 = __double2int_rz(yy);
-        const double dx0 = __dsub_rn(xx, (double)ix0), dy0 = __dsub_rn(yy, (double)iy0);
-        if (ix0 >= 0 && ix0 < w && iy0 >= 0 && iy0 < h) {
-            if (ix0 == w - 1 || iy0 == h - 1) {
-                pix = un[ix0 + (size_t)iy0 * w];
-            } else {
-                const double fac4 = __dmul_rn(dx0, dy0);
-                const size_t pos = ix0 + (size_t)iy0 * w;
-                const double v1 = un[pos], v3 = un[pos + w], v2 = un[pos + 1], v4 = un[pos + 1 + w];
-                const double w1 = __dadd_rn(__dsub_rn(__dsub_rn(1.0, dx0), dy0), fac4);
-                const double acc = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(v1, w1), __dmul_rn(v2, __dsub_rn(dx0, fac4))),
-                                                       __dmul_rn(v3, __dsub_rn(dy0, fac4))),
-                                             __dmul_rn(v4, fac4));
-                pix = __double2float_rn(acc);
-            }
-            if (normalize) pix = __double2float_rn(__ddiv_rn(__dsub_rn((double)pix, mean), sd));
-        } else if (fill == 1) {
-            pix = normalize ? 0.0f : __double2float_rn(mean);
-        } else if (fill == 2) {
-            pix = __int_as_float(0x7fc00000);
+    const float outside = fill == 1 ? (normalize ? 0.0f : __double2float_rn(mean))
+                          : fill == 2 ? __int_as_float(0x7fc00000) : 0.0f;
+    int f = 0;
+#pragma unroll
+    for (int q = 0; q < kAlignPix; q++) {
+        const size_t e = ((size_t)blockIdx.x * kAlignPix + q) * 256 + threadIdx.x;
+        if (e >= npix) break;
+        float pix;
+        bool in = true;
+        if (md == 1) {
+            pix = un[e];
         } else {
-            pix = 0.0f;
+            const int j = e >> 32 ? (int)(e / w) : (int)((unsigned)e / (unsigned)w), i = (int)(e - (size_t)j * w);
+            int st = 2;
+            if (md & 2) st = align_pixel_fixed(un, fix + 6 * t, md, i, j, w, h, &pix);
+            if (st == 2) in = align_pixel_exact(un, tinv + 6 * t, i, j, w, h, &pix);
+            else in = st == 1;
         }
+        if (!in) pix = outside;
+        else if (normalize) pix = __double2float_rn(__ddiv_rn(__dsub_rn((double)pix, mean), sd));
+        dst[e] = pix;
+        if (isnan(pix)) f |= 1;
+        else if (isinf(pix)) f |= 2;
     }
-    out[(size_t)t * w * h + (size_t)j * w + i] = pix;
+    f = __reduce_or_sync(0xffffffffu, f);
+    if ((threadIdx.x & 31) == 0 && f) atomicOr(flags, f);
 }
 
 // --- WBP row filter --------------------------------------------------------------
@@ -954,10 +1034,12 @@ cudaError_t launch_scan_nonfinite(const float* p, size_t n, int* flags, cudaStre
     return cudaGetLastError();
 }
 
-cudaError_t launch_align(const float* raw, float* out, const double* tinv, const double* stats, int N, int w, int h,
-                         int normalize, int fill, const unsigned char* identity, cudaStream_t s) {
-    dim3 grid((w + 127) / 128, h, N);
-    align_kernel<<<grid, 128, 0, s>>>(raw, out, tinv, stats, w, h, normalize, fill, identity);
+cudaError_t launch_align(const float* raw, float* out, const double* tinv, const long long* fix, const double* stats,
+                         int N, int w, int h, int normalize, int fill, const unsigned char* mode, int* flags,
+                         cudaStream_t s) {
+    const size_t npix = (size_t)w * h, per = 256 * kAlignPix;
+    align_kernel<<<dim3((unsigned)((npix + per - 1) / per), N), 256, 0, s>>>(raw, out, tinv, fix, stats, w, h, normalize,
+                                                                            fill, mode, flags);
     count_launch();
     return cudaGetLastError();
 }

@@ -723,6 +723,7 @@ tomo_status tomo_create(const tomo_geom* geom, const tomo_params* params, tomo_p
     A(alloc_n(p, &p->d_btilt, N));
     A(alloc_n(p, &p->d_zint, N * g.W));
     A(alloc_n(p, &p->d_tinv, N * 6));
+    A(alloc_n(p, &p->d_tfix, N * 6));
     A(alloc_n(p, &p->d_stats, N * 2));
     A(alloc_n(p, &p->d_identity, N));
     A(alloc_n(p, &p->d_mask, (size_t)g.w));
@@ -935,6 +936,7 @@ tomo_status tomo_load_series(tomo_projector* p, const float* pixels, int32_t pix
     CKS(setup_geometry(p));
     // alignment: Tinv = AffineTransform.createInverse (general case)
     std::vector<double> tinv((size_t)N * 6), st((size_t)N * 2);
+    std::vector<long long> tfix((size_t)N * 6);
     std::vector<unsigned char> ident(N);
     for (int t = 0; t < N; t++) {
         double T[6] = {1, 0, 0, 1, 0, 0};
@@ -951,17 +953,41 @@ tomo_status tomo_load_series(tomo_projector* p, const float* pixels, int32_t pix
         I[3] = m00 / det;
         I[4] = (m01 * m12 - m11 * m02) / det;
         I[5] = (m10 * m02 - m00 * m12) / det;
+        // fixed-point coordinates of pixel (i, j): (I00, I01) and (I10, I11) per column and row,
+        // the rest at (0, 0); used where every coordinate of the image stays below 2^14
+        const double cx = g.w / 2.0, cy = g.h / 2.0;
+        const double o[2] = {I[4] + cx - I[0] * cx - I[2] * cy, I[5] + cy - I[1] * cx - I[3] * cy};
+        long long* F = &tfix[6 * (size_t)t];
+        bool fits = true;
+        for (int k = 0; k < 2; k++) {
+            const double reach = std::fabs(I[k]) * g.w + std::fabs(I[2 + k]) * g.h + std::fabs(o[k]);
+            fits = fits && reach < 16384.0;  // false for NaN
+        }
+        for (int k = 0; k < 2 && fits; k++) {
+            F[k] = std::llrint(I[k] * 281474976710656.0);
+            F[2 + k] = std::llrint(I[2 + k] * 281474976710656.0);
+            F[4 + k] = std::llrint(o[k] * 281474976710656.0);
+        }
+        int mode = fits ? 2 : 0;
+        for (int k = 0; k < 2 && fits; k++) {
+            // multiples of 2^-20: the double expressions are exact too
+            const double s = 1048576.0;
+            if (I[k] * s == std::rint(I[k] * s) && I[2 + k] * s == std::rint(I[2 + k] * s) &&
+                I[4 + k] * s == std::rint(I[4 + k] * s))
+                mode |= 4 << k;
+        }
+        ident[t] = ident[t] ? 1 : (unsigned char)mode;
         st[2 * t] = stats ? stats[2 * t] : 0.0;
         st[2 * t + 1] = stats ? stats[2 * t + 1] : 1.0;
     }
     CK(cudaMemcpyAsync(p->d_tinv, tinv.data(), sizeof(double) * tinv.size(), cudaMemcpyHostToDevice, p->stream));
     CK(cudaMemcpyAsync(p->d_stats, st.data(), sizeof(double) * st.size(), cudaMemcpyHostToDevice, p->stream));
     CK(cudaMemcpyAsync(p->d_identity, ident.data(), N, cudaMemcpyHostToDevice, p->stream));
-    CK(launch_align(p->d_raw, p->d_meas, p->d_tinv, p->d_stats, N, g.w, g.h, p->params.normalize, p->params.fill,
-                    p->d_identity, p->stream));
+    CK(cudaMemcpyAsync(p->d_tfix, tfix.data(), sizeof(long long) * tfix.size(), cudaMemcpyHostToDevice, p->stream));
     int flags = 0;
     CK(cudaMemsetAsync(p->d_flags, 0, sizeof(int), p->stream));
-    CK(launch_scan_nonfinite(p->d_meas, (size_t)N * p->npix, p->d_flags, p->stream));
+    CK(launch_align(p->d_raw, p->d_meas, p->d_tinv, p->d_tfix, p->d_stats, N, g.w, g.h, p->params.normalize,
+                    p->params.fill, p->d_identity, p->d_flags, p->stream));
     CK(cudaMemcpyAsync(&flags, p->d_flags, sizeof(int), cudaMemcpyDeviceToHost, p->stream));
     CK(cudaStreamSynchronize(p->stream));
     p->meas_has_nan = (flags & 1) != 0;
@@ -1044,11 +1070,10 @@ tomo_status tomo_set_fill(tomo_projector* p, int32_t fill) {
     p->params.fill = fill;
     if (!p->series_loaded) return TOMO_OK;
     const Geometry& g = p->g;
-    CK(launch_align(p->d_raw, p->d_meas, p->d_tinv, p->d_stats, g.N, g.w, g.h, p->params.normalize, fill,
-                    p->d_identity, p->stream));
     int flags = 0;
     CK(cudaMemsetAsync(p->d_flags, 0, sizeof(int), p->stream));
-    CK(launch_scan_nonfinite(p->d_meas, (size_t)g.N * p->npix, p->d_flags, p->stream));
+    CK(launch_align(p->d_raw, p->d_meas, p->d_tinv, p->d_tfix, p->d_stats, g.N, g.w, g.h, p->params.normalize, fill,
+                    p->d_identity, p->d_flags, p->stream));
     CK(cudaMemcpyAsync(&flags, p->d_flags, sizeof(int), cudaMemcpyDeviceToHost, p->stream));
     CK(cudaStreamSynchronize(p->stream));
     p->meas_has_nan = (flags & 1) != 0;

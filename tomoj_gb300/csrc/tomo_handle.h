@@ -58,6 +58,7 @@ struct tomo_projector {
     double* d_euler = nullptr;               // generic geometry: [N][9] Euler matrices
     int32_t* d_zint = nullptr;
     double* d_tinv = nullptr;
+    long long* d_tfix = nullptr;  // the inverse transforms in fixed point (align_kernel)
     double* d_stats = nullptr;
     unsigned char* d_identity = nullptr;
     float* d_mask = nullptr;

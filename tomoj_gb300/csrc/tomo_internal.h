@@ -282,8 +282,11 @@ cudaError_t bp_init_attributes();
 // Image columns a BP tile may span for one tilt (segment pairs staged per tilt).
 int bp_segment_pairs(bool wide);
 
-cudaError_t launch_align(const float* raw, float* out, const double* tinv /*[N][6]*/, const double* stats, int N,
-                         int w, int h, int normalize, int fill, const unsigned char* identity, cudaStream_t s);
+// Aligned images (fix, mode: see align_kernel; |coordinates| below 2^14 for mode & 2); *flags
+// (zeroed by the caller) receives bit 0 for a NaN, bit 1 for an infinity among them.
+cudaError_t launch_align(const float* raw, float* out, const double* tinv /*[N][6]*/, const long long* fix /*[N][6]*/,
+                         const double* stats, int N, int w, int h, int normalize, int fill, const unsigned char* mode,
+                         int* flags, cudaStream_t s);
 // Row filters: bad (optional, one flag per image of rows_per_img rows) turns every row
 // of a flagged image into NaN, as the reference's 2-D transform does.
 cudaError_t launch_row_filter_tw(float* img, const float* mask_row, const float2* tw, int rows, int w,
