@@ -146,8 +146,203 @@ __global__ void __launch_bounds__(256) align_kernel(const float* __restrict__ ra
 // a mask that, for a zero tilt-axis angle, depends on the column frequency only;
 // the 2-D filter is then exactly a filter of every row.  Two real rows are packed
 // into one complex sequence (the mask is real and even, so the packed halves
-// stay separate), transformed by an in-shared-memory radix-2 FFT, multiplied by
-// the mask, transformed back and scaled by 1/w.
+// stay separate), transformed, multiplied by the mask, transformed back and scaled.
+//
+// Any width: the filter is a circular convolution of length w with the real kernel
+// h = IDFT_w(mask).  A row is laid out twice ([row, row], the periodic extension) in a
+// zero-padded sequence of M >= 2w - 1 points; the linear convolution with h (spectrum H,
+// M points) equals the circular one on outputs [w, 2w).
+//
+// One CTA per pair of rows; in-place passes of radix 8 (the first of 2, 4 or 8) over one
+// padded buffer in shared memory: decimation in frequency down to groups of 8 points,
+// which are transformed, multiplied by the spectrum (stored in the order the passes leave
+// it, fft_slot_frequency; twiddles in the order of use, fft_pass_twiddles) and transformed back in registers, then decimation in time back
+// up.  The first pass reads the image and the last one writes it, so M = 2048 crosses
+// shared memory 6 times each way and nothing is reordered; radix-2 stages with
+// bit-reversed copies crossed it 24 times.  Bound by shared memory and FP32 issue, about
+// evenly.  73 images of 750 x 333 (M = 2048): 881 -> 184 us; 61 of 512 x 256 (M = 512):
+// 121 -> 23 us (284 and 29 us with the twiddles gathered from one table by stride).
+__device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
+    return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+__device__ __forceinline__ float2 caddf(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ float2 csubf(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+// a * (-i) (forward) or a * i (inverse)
+template <bool INV>
+__device__ __forceinline__ float2 quarter(float2 a) {
+    return INV ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
+}
+
+// R-point transform in registers, outputs in natural order.
+template <int R, bool INV>
+__device__ __forceinline__ void fft_points(float2* v) {
+    if constexpr (R == 2) {
+        const float2 d = csubf(v[0], v[1]);
+        v[0] = caddf(v[0], v[1]);
+        v[1] = d;
+    } else if constexpr (R == 4) {
+        const float2 a = caddf(v[0], v[2]), b = csubf(v[0], v[2]);
+        const float2 c = caddf(v[1], v[3]), d = quarter<INV>(csubf(v[1], v[3]));
+        v[0] = caddf(a, c);
+        v[1] = caddf(b, d);
+        v[2] = csubf(a, c);
+        v[3] = csubf(b, d);
+    } else if constexpr (R == 8) {
+        float2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
+        fft_points<4, INV>(e);
+        fft_points<4, INV>(o);
+        const float r = 0.70710678118654752f;
+        const float2 q1 = quarter<INV>(o[1]), q3 = quarter<INV>(o[3]);
+        o[1] = make_float2(r * (o[1].x + q1.x), r * (o[1].y + q1.y));
+        o[2] = quarter<INV>(o[2]);
+        o[3] = make_float2(r * (q3.x - o[3].x), r * (q3.y - o[3].y));
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            v[k] = caddf(e[k], o[k]);
+            v[k + 4] = csubf(e[k], o[k]);
+        }
+    }
+}
+
+// Shared-memory place of point i: one spare place per 8 points keeps the accesses of a pass
+// with stride 1, 8 or >= 64 on different banks.
+__device__ __forceinline__ int fft_pad(int i) { return i + (i >> 3); }
+
+// One pass over groups of 2^logL points (sub-transforms of R points, stride 2^logL / R) of
+// an M-point sequence: load(i) and store(i, v) read and write point i.  Forward: transform,
+// then twiddles; inverse: twiddles, then transform.
+template <int R, bool INV, class Load, class Store>
+__device__ __forceinline__ void fft_pass(const float2* __restrict__ tw, int logM, int logL, Load load, Store store) {
+    constexpr int kLogR = R == 8 ? 3 : R == 4 ? 2 : R == 2 ? 1 : 0;
+    const int logS = logL - kLogR, cnt = 1 << (logM - kLogR);
+    for (int b = threadIdx.x; b < cnt; b += blockDim.x) {
+        const int k = b & ((1 << logS) - 1), i0 = ((b >> logS) << logL) + k;
+        float2 v[R];
+#pragma unroll
+        for (int m = 0; m < R; m++) v[m] = load(i0 + (m << logS));
+        if (!INV) fft_points<R, INV>(v);
+#pragma unroll
+        for (int m = 1; m < R; m++) {
+            float2 t = tw[(1 << logM) - (1 << logL) + ((m - 1) << logS) + k];
+            if (INV) t.y = -t.y;
+            v[m] = cmulf(v[m], t);
+        }
+        if (INV) fft_points<R, INV>(v);
+#pragma unroll
+        for (int m = 0; m < R; m++) store(i0 + (m << logS), v[m]);
+    }
+}
+
+// The groups of R contiguous points in between: transform, spectrum, inverse transform.
+template <int R, class Load, class Store, class Spec>
+__device__ __forceinline__ void fft_middle(int logM, Load load, Store store, Spec spec) {
+    constexpr int kLogR = R == 8 ? 3 : R == 4 ? 2 : R == 2 ? 1 : 0;
+    for (int b = threadIdx.x; b < 1 << (logM - kLogR); b += blockDim.x) {
+        float2 v[R];
+#pragma unroll
+        for (int m = 0; m < R; m++) v[m] = load(b * R + m);
+        fft_points<R, false>(v);
+#pragma unroll
+        for (int m = 0; m < R; m++) v[m] = spec(b * R + m, v[m]);
+        fft_points<R, true>(v);
+#pragma unroll
+        for (int m = 0; m < R; m++) store(b * R + m, v[m]);
+    }
+}
+
+// in(i): point i of the packed rows; out(i, v): point i of the filtered sequence times M.
+template <class In, class Out, class Spec>
+__device__ __forceinline__ void fft_filter(float2* s, const float2* __restrict__ tw, int logM, In in, Out out, Spec spec) {
+    auto ld = [s](int i) { return s[fft_pad(i)]; };
+    auto st = [s](int i, float2 v) { s[fft_pad(i)] = v; };
+    if (logM <= 3) {  // one group
+        if (logM == 3) fft_middle<8>(logM, in, out, spec);
+        else if (logM == 2) fft_middle<4>(logM, in, out, spec);
+        else if (logM == 1) fft_middle<2>(logM, in, out, spec);
+        else fft_middle<1>(logM, in, out, spec);
+        return;
+    }
+    const int first = logM % 3;
+    if (first == 1) fft_pass<2, false>(tw, logM, logM, in, st);
+    else if (first == 2) fft_pass<4, false>(tw, logM, logM, in, st);
+    else fft_pass<8, false>(tw, logM, logM, in, st);
+    const int top = logM - (first ? first : 3);
+    for (int l = top; l > 3; l -= 3) {
+        __syncthreads();
+        fft_pass<8, false>(tw, logM, l, ld, st);
+    }
+    __syncthreads();
+    fft_middle<8>(logM, ld, st, spec);
+    for (int l = 6; l <= top; l += 3) {
+        __syncthreads();
+        fft_pass<8, true>(tw, logM, l, ld, st);
+    }
+    __syncthreads();
+    if (first == 1) fft_pass<2, true>(tw, logM, logM, ld, out);
+    else if (first == 2) fft_pass<4, true>(tw, logM, logM, ld, out);
+    else fft_pass<8, true>(tw, logM, logM, ld, out);
+}
+
+// bad (optional): per-image flag of a non-finite pixel.  The reference's 2-D transform
+// spreads one NaN or Inf over the whole image; a row filter alone would keep it in
+// its row, so rows of a flagged image are written as NaN.
+__device__ __forceinline__ bool image_bad(const int* bad, int row, int rows_per_img) {
+    return bad != nullptr && bad[row / rows_per_img] != 0;
+}
+
+__global__ void __launch_bounds__(512) row_filter_kernel(float* img, const float* __restrict__ mask,
+                                                         const float2* __restrict__ tw, int rows, int n, int logn,
+                                                         const int* __restrict__ bad, int rows_per_img) {
+    extern __shared__ float2 sbuf[];
+    const int r0 = 2 * blockIdx.x, r1 = r0 + 1;
+    float* row0 = img + (size_t)r0 * n;
+    float* row1 = (r1 < rows) ? img + (size_t)r1 * n : nullptr;
+    const float inv = 1.0f / (float)n;
+    const bool bad0 = image_bad(bad, r0, rows_per_img), bad1 = row1 && image_bad(bad, r1, rows_per_img);
+    fft_filter(
+        sbuf, tw, logn, [=](int i) { return make_float2(row0[i], row1 ? row1[i] : 0.0f); },
+        [=](int i, float2 v) {
+            row0[i] = bad0 ? __int_as_float(0x7fc00000) : v.x * inv;
+            if (row1) row1[i] = bad1 ? __int_as_float(0x7fc00000) : v.y * inv;
+        },
+        [=](int i, float2 v) { return make_float2(v.x * mask[i], v.y * mask[i]); });
+}
+
+__global__ void __launch_bounds__(512) row_filter_conv_kernel(float* img, const float2* __restrict__ H,
+                                                              const float2* __restrict__ tw, int rows, int w, int M,
+                                                              int logM, const int* __restrict__ bad, int rows_per_img) {
+    extern __shared__ float2 sbuf[];
+    const int r0 = 2 * blockIdx.x, r1 = r0 + 1;
+    float* row0 = img + (size_t)r0 * w;
+    float* row1 = (r1 < rows) ? img + (size_t)r1 * w : nullptr;
+    const float inv = 1.0f / (float)M;
+    const bool bad0 = image_bad(bad, r0, rows_per_img), bad1 = row1 && image_bad(bad, r1, rows_per_img);
+    fft_filter(
+        sbuf, tw, logM,
+        [=](int i) {
+            if (i >= 2 * w) return make_float2(0.0f, 0.0f);
+            const int m = i < w ? i : i - w;
+            return make_float2(row0[m], row1 ? row1[m] : 0.0f);
+        },
+        [=](int i, float2 v) {
+            const int k = i - w;
+            if (k < 0 || k >= w) return;
+            row0[k] = bad0 ? __int_as_float(0x7fc00000) : v.x * inv;
+            if (row1) row1[k] = bad1 ? __int_as_float(0x7fc00000) : v.y * inv;
+        },
+        [=](int i, float2 v) { return cmulf(v, H[i]); });
+}
+
+// --- 2-D weighting (tilt axis not vertical) ----------------------------------------
+// FFTWeighting.weighting (FFTWeighting.java:87-112) with a mask that depends on both
+// frequencies: forward DFT of every row, transpose, per column (now a row) forward
+// DFT, multiply by the mask, inverse DFT, transpose back, inverse DFT of every row,
+// real part scaled by 1/(w h).  Each transform runs in shared memory: radix-2 when
+// the length is a power of two, otherwise Bluestein's chirp-z algorithm on a radix-2
+// grid of M >= 2n - 1 points:
+//   X[k] = c[k] * sum_j (x[j] c[j]) conj(c[k - j]),  c[j] = exp(-i pi j^2 / n),
+// the convolution done by an M-point FFT with the precomputed spectrum of the
+// wrapped conj(c).  Inverse transforms are conj(DFT(conj(x))).
 __device__ __forceinline__ unsigned bitrev(unsigned v, int bits) { return __brev(v) >> (32 - bits); }
 
 __device__ void fft_stages(float2* s, const float2* __restrict__ tw, int n, int logn, bool inverse) {
@@ -167,87 +362,6 @@ __device__ void fft_stages(float2* s, const float2* __restrict__ tw, int n, int 
         }
     }
     __syncthreads();
-}
-
-// bad (optional): per-image flag of a non-finite pixel.  The reference's 2-D transform
-// spreads one NaN or Inf over the whole image; a row filter alone would keep it in
-// its row, so rows of a flagged image are written as NaN.
-__device__ __forceinline__ bool image_bad(const int* bad, int row, int rows_per_img) {
-    return bad != nullptr && bad[row / rows_per_img] != 0;
-}
-
-__global__ void row_filter_kernel(float* img, const float* __restrict__ mask, const float2* __restrict__ tw, int rows,
-                                  int n, int logn, const int* __restrict__ bad, int rows_per_img) {
-    extern __shared__ float2 sbuf[];
-    float2* a = sbuf;
-    float2* b = sbuf + n;
-    const int r0 = 2 * blockIdx.x, r1 = r0 + 1;
-    float* row0 = img + (size_t)r0 * n;
-    float* row1 = (r1 < rows) ? img + (size_t)r1 * n : nullptr;
-    for (int k = threadIdx.x; k < n; k += blockDim.x)
-        a[bitrev(k, logn)] = make_float2(row0[k], row1 ? row1[k] : 0.0f);
-    fft_stages(a, tw, n, logn, false);
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        const float m = mask[k];
-        const float2 v = a[k];
-        b[bitrev(k, logn)] = make_float2(v.x * m, v.y * m);
-    }
-    fft_stages(b, tw, n, logn, true);
-    const float inv = 1.0f / (float)n;
-    const bool bad0 = image_bad(bad, r0, rows_per_img), bad1 = row1 && image_bad(bad, r1, rows_per_img);
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        row0[k] = bad0 ? __int_as_float(0x7fc00000) : b[k].x * inv;
-        if (row1) row1[k] = bad1 ? __int_as_float(0x7fc00000) : b[k].y * inv;
-    }
-}
-
-// Any width: the row filter is a circular convolution of length w with the real
-// kernel h = IDFT_w(mask).  Rows are laid out twice ([row, row], the periodic
-// extension) in a zero-padded power-of-two buffer of M >= 2w - 1 points; the linear
-// convolution with h (spectrum H, M points) equals the circular one on outputs
-// [w, 2w).  Two real rows are packed into one complex sequence as above (h is real).
-__global__ void row_filter_conv_kernel(float* img, const float2* __restrict__ H, const float2* __restrict__ tw, int rows,
-                                       int w, int M, int logM, const int* __restrict__ bad, int rows_per_img) {
-    extern __shared__ float2 sbuf[];
-    float2* a = sbuf;
-    const int r0 = 2 * blockIdx.x, r1 = r0 + 1;
-    float* row0 = img + (size_t)r0 * w;
-    float* row1 = (r1 < rows) ? img + (size_t)r1 * w : nullptr;
-    for (int k = threadIdx.x; k < M; k += blockDim.x) {
-        float2 v = make_float2(0.0f, 0.0f);
-        if (k < 2 * w) {
-            const int m = k < w ? k : k - w;
-            v = make_float2(row0[m], row1 ? row1[m] : 0.0f);
-        }
-        a[bitrev(k, logM)] = v;
-    }
-    fft_stages(a, tw, M, logM, false);
-    float2* b = sbuf + M;
-    for (int k = threadIdx.x; k < M; k += blockDim.x) {
-        const float2 v = a[k], f = H[k];
-        b[bitrev(k, logM)] = make_float2(v.x * f.x - v.y * f.y, v.x * f.y + v.y * f.x);
-    }
-    fft_stages(b, tw, M, logM, true);
-    const float inv = 1.0f / (float)M;
-    const bool bad0 = image_bad(bad, r0, rows_per_img), bad1 = row1 && image_bad(bad, r1, rows_per_img);
-    for (int k = threadIdx.x; k < w; k += blockDim.x) {
-        row0[k] = bad0 ? __int_as_float(0x7fc00000) : b[w + k].x * inv;
-        if (row1) row1[k] = bad1 ? __int_as_float(0x7fc00000) : b[w + k].y * inv;
-    }
-}
-
-// --- 2-D weighting (tilt axis not vertical) ----------------------------------------
-// FFTWeighting.weighting (FFTWeighting.java:87-112) with a mask that depends on both
-// frequencies: forward DFT of every row, transpose, per column (now a row) forward
-// DFT, multiply by the mask, inverse DFT, transpose back, inverse DFT of every row,
-// real part scaled by 1/(w h).  Each transform runs in shared memory: radix-2 when
-// the length is a power of two, otherwise Bluestein's chirp-z algorithm on a radix-2
-// grid of M >= 2n - 1 points:
-//   X[k] = c[k] * sum_j (x[j] c[j]) conj(c[k - j]),  c[j] = exp(-i pi j^2 / n),
-// the convolution done by an M-point FFT with the precomputed spectrum of the
-// wrapped conj(c).  Inverse transforms are conj(DFT(conj(x))).
-__device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
-    return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
 // Forward DFT (conjugated on input and output when conj_io: the inverse) of x[0, n)
@@ -981,12 +1095,15 @@ __global__ void scan_nonfinite_kernel(const float* __restrict__ p, size_t n, int
 
 }  // namespace
 
+static size_t row_filter_smem(int M) { return (size_t)(M + M / 8 + 1) * sizeof(float2); }
+static int row_filter_threads(int M) { return std::min(std::max(M / 8, 32), 512); }
+
 cudaError_t misc_init_attributes() {
     cudaError_t e = cudaFuncSetAttribute(row_filter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         2 * 4096 * (int)sizeof(float2));
+                                         (int)row_filter_smem(4096));
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(row_filter_conv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             2 * kRowConvMaxM * (int)sizeof(float2));
+                             (int)row_filter_smem(kRowConvMaxM));
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(tv_step4_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTv4Smem);
     if (e != cudaSuccess) return e;
@@ -1049,8 +1166,7 @@ cudaError_t launch_row_filter_tw(float* img, const float* mask_row, const float2
     int logn = 0;
     while ((1 << logn) < w) logn++;
     if ((1 << logn) != w) return cudaErrorInvalidValue;
-    const size_t smem = 2 * (size_t)w * sizeof(float2);
-    row_filter_kernel<<<(rows + 1) / 2, 256, smem, s>>>(img, mask_row, tw, rows, w, logn, bad, rows_per_img);
+    row_filter_kernel<<<(rows + 1) / 2, row_filter_threads(w), row_filter_smem(w), s>>>(img, mask_row, tw, rows, w, logn, bad, rows_per_img);
     count_launch();
     return cudaGetLastError();
 }
@@ -1060,8 +1176,7 @@ cudaError_t launch_row_filter_conv(float* img, const float2* H, const float2* tw
     int logM = 0;
     while ((1 << logM) < M) logM++;
     if ((1 << logM) != M || M < 2 * w - 1 || M > kRowConvMaxM) return cudaErrorInvalidValue;
-    const size_t smem = 2 * (size_t)M * sizeof(float2);
-    row_filter_conv_kernel<<<(rows + 1) / 2, 256, smem, s>>>(img, H, tw, rows, w, M, logM, bad, rows_per_img);
+    row_filter_conv_kernel<<<(rows + 1) / 2, row_filter_threads(M), row_filter_smem(M), s>>>(img, H, tw, rows, w, M, logM, bad, rows_per_img);
     count_launch();
     return cudaGetLastError();
 }

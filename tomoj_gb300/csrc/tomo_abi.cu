@@ -1436,15 +1436,13 @@ tomo_status tomo_set_weighting(tomo_projector* p, int32_t kind, double radius, c
     weighting_row_filter(kind, g.w, g.N, sint.data(), deg.data(), radius * g.w, mask.data());
     if ((g.w & (g.w - 1)) != 0) {
         // any width: circular convolution with h = IDFT_w(mask) through an M-point FFT
-        int M = 1;
-        while (M < 2 * g.w - 1) M <<= 1;
+        int M = 1, logM = 0;
+        while (M < 2 * g.w - 1) M <<= 1, logM++;
         if (M > kRowConvMaxM) return fail(TOMO_ERR_UNSUPPORTED, "weighting supports widths up to 4096");
-        std::vector<float2> H(M), twm(M);
-        row_filter_spectrum(mask.data(), g.w, M, H.data());
-        for (int k = 0; k < M; k++) {
-            const double a = -2.0 * M_PI * k / M;
-            twm[k] = make_float2((float)std::cos(a), (float)std::sin(a));
-        }
+        std::vector<float2> Hn(M), H(M), twm(M);
+        row_filter_spectrum(mask.data(), g.w, M, Hn.data());
+        for (int k = 0; k < M; k++) H[k] = Hn[fft_slot_frequency(k, logM)];
+        fft_pass_twiddles(logM, twm.data());
         if (p->conv_M < M) {
             CKS(alloc_n(p, &p->d_convH, (size_t)M));
             CKS(alloc_n(p, &p->d_convTw, (size_t)M));
@@ -1457,11 +1455,12 @@ tomo_status tomo_set_weighting(tomo_projector* p, int32_t kind, double radius, c
         return TOMO_OK;
     }
     std::vector<float2> tw(g.w);
-    for (int k = 0; k < g.w; k++) {
-        const double a = -2.0 * M_PI * k / g.w;
-        tw[k] = make_float2((float)std::cos(a), (float)std::sin(a));
-    }
-    CK(cudaMemcpyAsync(p->d_mask, mask.data(), sizeof(float) * g.w, cudaMemcpyHostToDevice, p->stream));
+    int logw = 0;
+    while ((1 << logw) < g.w) logw++;
+    fft_pass_twiddles(logw, tw.data());
+    std::vector<float> order(g.w);
+    for (int k = 0; k < g.w; k++) order[k] = mask[fft_slot_frequency(k, logw)];
+    CK(cudaMemcpyAsync(p->d_mask, order.data(), sizeof(float) * g.w, cudaMemcpyHostToDevice, p->stream));
     CK(cudaMemcpyAsync(p->d_tw, tw.data(), sizeof(float2) * g.w, cudaMemcpyHostToDevice, p->stream));
     CK(cudaStreamSynchronize(p->stream));
     p->weight_kind = kind;

@@ -11,6 +11,7 @@
 // exact double arithmetic and shipped as per-ray / per-column z intervals.
 #pragma once
 #include <atomic>
+#include <cmath>
 #include <functional>
 #include <vector>
 #include <cstddef>
@@ -287,8 +288,32 @@ int bp_segment_pairs(bool wide);
 cudaError_t launch_align(const float* raw, float* out, const double* tinv /*[N][6]*/, const long long* fix /*[N][6]*/,
                          const double* stats, int N, int w, int h, int normalize, int fill, const unsigned char* mode,
                          int* flags, cudaStream_t s);
-// Row filters: bad (optional, one flag per image of rows_per_img rows) turns every row
+// Row filters: mask_row and H lie in the order in which the in-place passes leave the
+// spectrum (slot i holds frequency fft_slot_frequency(i, log2 of the length)); the first pass
+// takes log2 mod 3 bits (3 when that is 0), the others 3.  bad (optional, one flag per image of rows_per_img rows) turns every row
 // of a flagged image into NaN, as the reference's 2-D transform does.
+inline int fft_slot_frequency(int slot, int logn) {
+    int f = 0, done = 0;
+    for (int left = logn, b = logn % 3 ? logn % 3 : 3; left > 0; left -= b, b = 3) {
+        if (b > left) b = left;
+        f |= ((slot >> (left - b)) & ((1 << b) - 1)) << done;
+        done += b;
+    }
+    return f;
+}
+// Their twiddles exp(-2 pi i m k / L), pass after pass: for a pass over groups of L points with
+// radix R, m = 1 .. R - 1 rows of L / R entries k, from place n - L on.
+inline void fft_pass_twiddles(int logn, float2* tw) {
+    const int n = 1 << logn;
+    for (int logl = logn, b = logn % 3 ? logn % 3 : 3; logl > 3; logl -= b, b = 3) {
+        const int L = 1 << logl, S = L >> b;
+        for (int m = 1; m < 1 << b; m++)
+            for (int k = 0; k < S; k++) {
+                const double a = -2.0 * M_PI * ((double)m * k) / L;
+                tw[n - L + (m - 1) * S + k] = make_float2((float)std::cos(a), (float)std::sin(a));
+            }
+    }
+}
 cudaError_t launch_row_filter_tw(float* img, const float* mask_row, const float2* tw, int rows, int w,
                                  const int* bad, int rows_per_img, cudaStream_t s);
 // Row filter of any width as a circular convolution (spectrum H and twiddles of M points,
