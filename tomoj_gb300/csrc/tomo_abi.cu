@@ -314,9 +314,11 @@ tomo_status launch_fp(tomo_projector* p, FpLaunch a, bool whole = false) {
     return TOMO_OK;
 }
 
-// Forward projection of the current batch, with the fused difference when meas is given.
+// Forward projection of the current batch, with the fused difference when meas is given.  `reduce`:
+// also sum the squared errors of these T tilts (an iteration over many subsets sums all of them once
+// at its end: each slot keeps its rows' sums in d_errpart).
 tomo_status run_fp(tomo_projector* p, const int* d_tilts, int T, int y0, bool with_diff, double factor,
-                   int slot0) {
+                   int slot0, bool reduce = true) {
     const Geometry& g = p->g;
     int j0, j1;
     fp_rows(p, y0, &j0, &j1);
@@ -367,7 +369,7 @@ tomo_status run_fp(tomo_projector* p, const int* d_tilts, int T, int y0, bool wi
         if (p->params.long_object) CK(launch_long_object(norm, T, g.h, g.w, p->stream));
         if (with_diff) {
             CK(launch_diff(p->d_meas, d_tilts, proj, norm, diff, errpart, T, g.w, g.h, j0, j1, factor, p->stream));
-            CK(launch_reduce_err(errpart, p->d_err + slot0, T, g.h, p->stream));
+            if (reduce) CK(launch_reduce_err(errpart, p->d_err + slot0, T, g.h, p->stream));
         }
         return TOMO_OK;
     }
@@ -407,7 +409,7 @@ tomo_status run_fp(tomo_projector* p, const int* d_tilts, int T, int y0, bool wi
         if (with_diff)
             CK(launch_diff(p->d_meas, d_tilts, proj, norm, diff, errpart, T, g.w, g.h, j0, j1, factor, p->stream));
     }
-    if (with_diff) CK(launch_reduce_err(errpart, p->d_err + slot0, T, g.h, p->stream));
+    if (with_diff && reduce) CK(launch_reduce_err(errpart, p->d_err + slot0, T, g.h, p->stream));
     return TOMO_OK;
 }
 
@@ -1919,6 +1921,8 @@ tomo_status tomo_run_ossart(tomo_projector* p, int32_t n_iter, double relax, int
                 CK(cudaStreamBeginCapture(p->stream, cudaStreamCaptureModeThreadLocal));
                 tomo_status bs = body(d_cur);
                 cudaError_t ce = cudaStreamEndCapture(p->stream, &graph);
+        // rj0 >= rj1: nothing was projected and d_err keeps its values
+        if (rj0 < rj1) CK(launch_reduce_err(p->d_errpart, p->d_err, N, g.h, p->stream));
                 // kernels are counted when the graph runs, not when it is captured
                 graph_kernels = tomo::g_launches.load() - before;
                 tomo::g_launches -= graph_kernels;
