@@ -1897,7 +1897,7 @@ tomo_status tomo_run_ossart(tomo_projector* p, int32_t n_iter, double relax, int
         for (int s = 0, k = 0; s < N; s += upd, k++) {
             const int T = std::min(upd, N - s);
             if (p->profile) CK(cudaEventRecordWithFlags(p->ev[4 * k + 0], p->stream, cudaEventRecordExternal));
-            CKS(run_fp(p, d_ord + s, T, y0, true, factor, s));
+            CKS(run_fp(p, d_ord + s, T, y0, true, factor, s, false));
             if (p->profile) CK(cudaEventRecordWithFlags(p->ev[4 * k + 1], p->stream, cudaEventRecordExternal));
             CKS(run_bp(p, p->d_diff + (size_t)s * p->npix, d_ord + s, T, y0, y1, p->meas_has_inf, true));
             if (p->profile) CK(cudaEventRecordWithFlags(p->ev[4 * k + 2], p->stream, cudaEventRecordExternal));
