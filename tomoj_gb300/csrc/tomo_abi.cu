@@ -1902,6 +1902,8 @@ tomo_status tomo_run_ossart(tomo_projector* p, int32_t n_iter, double relax, int
             CKS(run_bp(p, p->d_diff + (size_t)s * p->npix, d_ord + s, T, y0, y1, p->meas_has_inf, true));
             if (p->profile) CK(cudaEventRecordWithFlags(p->ev[4 * k + 2], p->stream, cudaEventRecordExternal));
         }
+        // rj0 >= rj1: nothing was projected and d_err keeps its values
+        if (rj0 < rj1) CK(launch_reduce_err(p->d_errpart, p->d_err, N, g.h, p->stream));
         CKS(end_iteration(p));
         return TOMO_OK;
     };
@@ -1921,8 +1923,6 @@ tomo_status tomo_run_ossart(tomo_projector* p, int32_t n_iter, double relax, int
                 CK(cudaStreamBeginCapture(p->stream, cudaStreamCaptureModeThreadLocal));
                 tomo_status bs = body(d_cur);
                 cudaError_t ce = cudaStreamEndCapture(p->stream, &graph);
-        // rj0 >= rj1: nothing was projected and d_err keeps its values
-        if (rj0 < rj1) CK(launch_reduce_err(p->d_errpart, p->d_err, N, g.h, p->stream));
                 // kernels are counted when the graph runs, not when it is captured
                 graph_kernels = tomo::g_launches.load() - before;
                 tomo::g_launches -= graph_kernels;
