@@ -97,7 +97,7 @@ __device__ __forceinline__ int align_pixel_fixed(const float* __restrict__ un, c
 // mode per image: 0 double expressions, 1 identity, 2 fixed-point coordinates (fix: {x, y per
 // column, x, y per row, x, y at pixel (0, 0)} times 2^48) with + 4 and + 8 where x and y are
 // exact in both forms (whole or dyadic shifts).  flags: bit 0 a NaN was written, bit 1 an
-// infinity.  This part's FP64 rate is 1/64 of FP32: 61 images of 512 x 256 took 628
+// infinity, bit 2 set where a pixel took the fill.  This part's FP64 rate is 1/64 of FP32: 61 images of 512 x 256 took 628
 // us in doubles and take 65 us in fixed point and float pairs, with the scan for
 // non-finite pixels (9 us) in the same pass.
 constexpr int kAlignPix = 4;  // pixels per thread
@@ -131,8 +131,12 @@ __global__ void __launch_bounds__(256) align_kernel(const float* __restrict__ ra
             if (st == 2) in = align_pixel_exact(un, tinv + 6 * t, i, j, w, h, &pix);
             else in = st == 1;
         }
-        if (!in) pix = outside;
-        else if (normalize) pix = __double2float_rn(__ddiv_rn(__dsub_rn((double)pix, mean), sd));
+        if (!in) {
+            pix = outside;
+            f |= 4;
+        } else if (normalize) {
+            pix = __double2float_rn(__ddiv_rn(__dsub_rn((double)pix, mean), sd));
+        }
         dst[e] = pix;
         if (isnan(pix)) f |= 1;
         else if (isinf(pix)) f |= 2;
@@ -290,17 +294,28 @@ __device__ __forceinline__ bool image_bad(const int* bad, int row, int rows_per_
     return bad != nullptr && bad[row / rows_per_img] != 0;
 }
 
-__global__ void __launch_bounds__(512) row_filter_kernel(float* img, const float* __restrict__ mask,
-                                                         const float2* __restrict__ tw, int rows, int n, int logn,
-                                                         const int* __restrict__ bad, int rows_per_img) {
+// Row of the source of filtered row r: img itself, or the row of image pick[r / rows_per_img] of src.
+__device__ __forceinline__ const float* source_row(const float* img, const float* src, const int* pick, int r, int w,
+                                                   int rows_per_img) {
+    if (!src) return img + (size_t)r * w;
+    const int t = r / rows_per_img;
+    return src + ((size_t)pick[t] * rows_per_img + (r - t * rows_per_img)) * w;
+}
+
+__global__ void __launch_bounds__(512) row_filter_kernel(float* img, const float* src, const int* pick,
+                                                         const float* __restrict__ mask, const float2* __restrict__ tw,
+                                                         int rows, int n, int logn, const int* __restrict__ bad,
+                                                         int rows_per_img) {
     extern __shared__ float2 sbuf[];
     const int r0 = 2 * blockIdx.x, r1 = r0 + 1;
     float* row0 = img + (size_t)r0 * n;
     float* row1 = (r1 < rows) ? img + (size_t)r1 * n : nullptr;
+    const float* in0 = source_row(img, src, pick, r0, n, rows_per_img);
+    const float* in1 = row1 ? source_row(img, src, pick, r1, n, rows_per_img) : nullptr;
     const float inv = 1.0f / (float)n;
     const bool bad0 = image_bad(bad, r0, rows_per_img), bad1 = row1 && image_bad(bad, r1, rows_per_img);
     fft_filter(
-        sbuf, tw, logn, [=](int i) { return make_float2(row0[i], row1 ? row1[i] : 0.0f); },
+        sbuf, tw, logn, [=](int i) { return make_float2(in0[i], in1 ? in1[i] : 0.0f); },
         [=](int i, float2 v) {
             row0[i] = bad0 ? __int_as_float(0x7fc00000) : v.x * inv;
             if (row1) row1[i] = bad1 ? __int_as_float(0x7fc00000) : v.y * inv;
@@ -308,13 +323,16 @@ __global__ void __launch_bounds__(512) row_filter_kernel(float* img, const float
         [=](int i, float2 v) { return make_float2(v.x * mask[i], v.y * mask[i]); });
 }
 
-__global__ void __launch_bounds__(512) row_filter_conv_kernel(float* img, const float2* __restrict__ H,
+__global__ void __launch_bounds__(512) row_filter_conv_kernel(float* img, const float* src, const int* pick,
+                                                              const float2* __restrict__ H,
                                                               const float2* __restrict__ tw, int rows, int w, int M,
                                                               int logM, const int* __restrict__ bad, int rows_per_img) {
     extern __shared__ float2 sbuf[];
     const int r0 = 2 * blockIdx.x, r1 = r0 + 1;
     float* row0 = img + (size_t)r0 * w;
     float* row1 = (r1 < rows) ? img + (size_t)r1 * w : nullptr;
+    const float* in0 = source_row(img, src, pick, r0, w, rows_per_img);
+    const float* in1 = row1 ? source_row(img, src, pick, r1, w, rows_per_img) : nullptr;
     const float inv = 1.0f / (float)M;
     const bool bad0 = image_bad(bad, r0, rows_per_img), bad1 = row1 && image_bad(bad, r1, rows_per_img);
     fft_filter(
@@ -322,7 +340,7 @@ __global__ void __launch_bounds__(512) row_filter_conv_kernel(float* img, const 
         [=](int i) {
             if (i >= 2 * w) return make_float2(0.0f, 0.0f);
             const int m = i < w ? i : i - w;
-            return make_float2(row0[m], row1 ? row1[m] : 0.0f);
+            return make_float2(in0[m], in1 ? in1[m] : 0.0f);
         },
         [=](int i, float2 v) {
             const int k = i - w;
@@ -1161,22 +1179,22 @@ cudaError_t launch_align(const float* raw, float* out, const double* tinv, const
     return cudaGetLastError();
 }
 
-cudaError_t launch_row_filter_tw(float* img, const float* mask_row, const float2* tw, int rows, int w,
+cudaError_t launch_row_filter_tw(float* img, const float* src, const int* pick, const float* mask_row, const float2* tw, int rows, int w,
                                  const int* bad, int rows_per_img, cudaStream_t s) {
     int logn = 0;
     while ((1 << logn) < w) logn++;
     if ((1 << logn) != w) return cudaErrorInvalidValue;
-    row_filter_kernel<<<(rows + 1) / 2, row_filter_threads(w), row_filter_smem(w), s>>>(img, mask_row, tw, rows, w, logn, bad, rows_per_img);
+    row_filter_kernel<<<(rows + 1) / 2, row_filter_threads(w), row_filter_smem(w), s>>>(img, src, pick, mask_row, tw, rows, w, logn, bad, rows_per_img);
     count_launch();
     return cudaGetLastError();
 }
 
-cudaError_t launch_row_filter_conv(float* img, const float2* H, const float2* tw, int rows, int w, int M,
-                                   const int* bad, int rows_per_img, cudaStream_t s) {
+cudaError_t launch_row_filter_conv(float* img, const float* src, const int* pick, const float2* H, const float2* tw,
+                                   int rows, int w, int M, const int* bad, int rows_per_img, cudaStream_t s) {
     int logM = 0;
     while ((1 << logM) < M) logM++;
     if ((1 << logM) != M || M < 2 * w - 1 || M > kRowConvMaxM) return cudaErrorInvalidValue;
-    row_filter_conv_kernel<<<(rows + 1) / 2, row_filter_threads(M), row_filter_smem(M), s>>>(img, H, tw, rows, w, M, logM, bad, rows_per_img);
+    row_filter_conv_kernel<<<(rows + 1) / 2, row_filter_threads(M), row_filter_smem(M), s>>>(img, src, pick, H, tw, rows, w, M, logM, bad, rows_per_img);
     count_launch();
     return cudaGetLastError();
 }

@@ -463,11 +463,28 @@ tomo_status apply_weighting(tomo_projector* p, float* imgs, int T) {
         float* im = imgs + (size_t)t0 * p->npix;
         CK(launch_image_nonfinite(im, tc, p->npix, p->d_imgbad, p->stream));
         if (p->conv_M > 0)
-            CK(launch_row_filter_conv(im, p->d_convH, p->d_convTw, tc * g.h, g.w, p->conv_M, p->d_imgbad, g.h,
+            CK(launch_row_filter_conv(im, nullptr, nullptr, p->d_convH, p->d_convTw, tc * g.h, g.w, p->conv_M, p->d_imgbad, g.h,
                                       p->stream));
         else
-            CK(launch_row_filter_tw(im, p->d_mask, p->d_tw, tc * g.h, g.w, p->d_imgbad, g.h, p->stream));
+            CK(launch_row_filter_tw(im, nullptr, nullptr, p->d_mask, p->d_tw, tc * g.h, g.w, p->d_imgbad, g.h, p->stream));
     }
+    return TOMO_OK;
+}
+
+// d_obatch = the measured images d_batch[0 .. T), weighted; `copied`: it holds them already.  The row filter reads a
+// series without NaN or Inf directly (no copy, no scan of the copies).
+tomo_status weighted_batch(tomo_projector* p, int T, bool copied) {
+    const Geometry& g = p->g;
+    if (p->weight_kind == TOMO_WEIGHT_NONE || p->weight2d || copied || p->meas_has_nan || p->meas_has_inf || T <= 0) {
+        if (!copied) CK(launch_gather(p->d_obatch, p->d_meas, p->d_batch, T, p->npix, p->stream));
+        return apply_weighting(p, p->d_obatch, T);
+    }
+    if (p->conv_M > 0)
+        CK(launch_row_filter_conv(p->d_obatch, p->d_meas, p->d_batch, p->d_convH, p->d_convTw, T * g.h, g.w, p->conv_M,
+                                  nullptr, g.h, p->stream));
+    else
+        CK(launch_row_filter_tw(p->d_obatch, p->d_meas, p->d_batch, p->d_mask, p->d_tw, T * g.h, g.w, nullptr, g.h,
+                                p->stream));
     return TOMO_OK;
 }
 
@@ -994,6 +1011,7 @@ tomo_status tomo_load_series(tomo_projector* p, const float* pixels, int32_t pix
     CK(cudaStreamSynchronize(p->stream));
     p->meas_has_nan = (flags & 1) != 0;
     p->meas_has_inf = (flags & 2) != 0;
+    p->meas_filled = (flags & 4) != 0;
     p->series_loaded = true;
     p->batch.clear();
     p->batch_uploaded = false;
@@ -1071,6 +1089,10 @@ tomo_status tomo_set_fill(tomo_projector* p, int32_t fill) {
     if (fill < TOMO_FILL_NONE || fill > TOMO_FILL_NAN) return fail(TOMO_ERR_INVALID, "unknown fill type");
     p->params.fill = fill;
     if (!p->series_loaded) return TOMO_OK;
+    if (!p->meas_filled) {  // no aligned pixel lies outside its image: every fill gives these
+        p->obatch_valid = false;
+        return TOMO_OK;
+    }
     const Geometry& g = p->g;
     int flags = 0;
     CK(cudaMemsetAsync(p->d_flags, 0, sizeof(int), p->stream));
@@ -1080,6 +1102,7 @@ tomo_status tomo_set_fill(tomo_projector* p, int32_t fill) {
     CK(cudaStreamSynchronize(p->stream));
     p->meas_has_nan = (flags & 1) != 0;
     p->meas_has_inf = (flags & 2) != 0;
+    p->meas_filled = (flags & 4) != 0;
     p->obatch_valid = false;
     return TOMO_OK;
 }
@@ -1301,11 +1324,8 @@ tomo_status tomo_backproject(tomo_projector* p, int32_t y0, int32_t y1) {
         imgs = p->d_diff;
         sanitize = p->meas_has_inf;
     } else {
-        if (!p->obatch_valid) {
-            CK(launch_gather(p->d_obatch, p->d_meas, p->d_batch, T, p->npix, p->stream));
-            p->obatch_valid = true;
-        }
-        CKS(apply_weighting(p, p->d_obatch, T));
+        CKS(weighted_batch(p, T, p->obatch_valid));
+        p->obatch_valid = true;
         imgs = p->d_obatch;
         sanitize = p->meas_has_nan || p->meas_has_inf;
     }
@@ -1758,8 +1778,7 @@ tomo_status tomo_run_wbp(tomo_projector* p, int32_t y0, int32_t y1) {
     std::vector<int> all(N);
     for (int t = 0; t < N; t++) all[t] = t;
     CK(cudaMemcpyAsync(p->d_batch, all.data(), sizeof(int) * N, cudaMemcpyHostToDevice, p->stream));
-    CK(launch_gather(p->d_obatch, p->d_meas, p->d_batch, N, p->npix, p->stream));
-    CKS(apply_weighting(p, p->d_obatch, N));
+    CKS(weighted_batch(p, N, false));
     CKS(run_bp(p, p->d_obatch, p->d_batch, N, y0, y1, p->meas_has_nan || p->meas_has_inf, false));
     CKS(check_status(p));
     p->batch.clear();

@@ -87,6 +87,7 @@ struct tomo_projector {
     bool projected = false;
     bool obatch_valid = false;
     bool meas_has_nan = false, meas_has_inf = false;
+    bool meas_filled = true;  // an aligned pixel took the fill value
     bool vol_nonfinite = false;
     // the flag of the volume this handle works on (the owner's when shared)
     bool& vol_flag() { return vol_owner ? vol_owner->vol_nonfinite : vol_nonfinite; }

@@ -284,7 +284,8 @@ cudaError_t bp_init_attributes();
 int bp_segment_pairs(bool wide);
 
 // Aligned images (fix, mode: see align_kernel; |coordinates| below 2^14 for mode & 2); *flags
-// (zeroed by the caller) receives bit 0 for a NaN, bit 1 for an infinity among them.
+// (zeroed by the caller) receives bit 0 for a NaN, bit 1 for an infinity among them, bit 2 where a
+// pixel took the fill.
 cudaError_t launch_align(const float* raw, float* out, const double* tinv /*[N][6]*/, const long long* fix /*[N][6]*/,
                          const double* stats, int N, int w, int h, int normalize, int fill, const unsigned char* mode,
                          int* flags, cudaStream_t s);
@@ -314,13 +315,14 @@ inline void fft_pass_twiddles(int logn, float2* tw) {
             }
     }
 }
-cudaError_t launch_row_filter_tw(float* img, const float* mask_row, const float2* tw, int rows, int w,
+// With src, image t of the filtered rows is made from image pick[t] of src instead of in place.
+cudaError_t launch_row_filter_tw(float* img, const float* src, const int* pick, const float* mask_row, const float2* tw, int rows, int w,
                                  const int* bad, int rows_per_img, cudaStream_t s);
 // Row filter of any width as a circular convolution (spectrum H and twiddles of M points,
 // M a power of two >= 2w - 1, at most kRowConvMaxM).
 constexpr int kRowConvMaxM = 8192;
-cudaError_t launch_row_filter_conv(float* img, const float2* H, const float2* tw, int rows, int w, int M,
-                                   const int* bad, int rows_per_img, cudaStream_t s);
+cudaError_t launch_row_filter_conv(float* img, const float* src, const int* pick, const float2* H, const float2* tw,
+                                   int rows, int w, int M, const int* bad, int rows_per_img, cudaStream_t s);
 // bad[t] = 1 when image t (npix floats) holds a NaN or an Inf, else 0.
 cudaError_t launch_image_nonfinite(const float* imgs, int T, size_t npix, int* bad, cudaStream_t s);
 // One DFT length for the 2-D weighting: radix-2 when n is a power of two (M == n),
