@@ -378,8 +378,14 @@ __global__ void __launch_bounds__(kBpCtaThreads, BpOcc<VT>::value)
 //
 // Tile: 64 x-columns x 4*KZ z-planes x 2 rows; thread (tx, tzg) owns KZ voxels along z of
 // column x0 + tx in both rows.  16 tilts are staged per chunk.  16-bit volumes take the
-// per-chunk Kahan form only (no per-add NaN / positivity rules: those go to the one-row
-// kernel).
+// chunked Kahan form only (no per-add NaN / positivity rules: those go to the one-row
+// kernel), with the one-row kernel's sums of 32 tilts and its order of adds, so the result
+// is bitwise the same.  Their registers hold the running sum alone: the voxel is read at the
+// end, and the first sum of more than 32 tilts waits in shared memory, so 16 voxels per row
+// and three CTAs per SM remain.  Up to 64 tilts: further sums would need compensations in
+// shared memory and leave two CTAs (2048 x 256 x 512, 121 tilts: 10.5 ms either way).
+// 1024 x 1024 x 256 in FP16: 5506 us with one row per thread, 4397 us with two for 61
+// tilts; 1178 and 825 us for 7.
 template <int KZ>
 struct Bp2 {
     static constexpr int kTC = 16;
@@ -392,18 +398,18 @@ struct Bp2 {
     static constexpr size_t az_off = zint_off + sizeof(int) * kTC * kTX;                 // long long [kTC][4]
     static constexpr size_t cs_off = az_off + sizeof(long long) * kTC * 4;               // long long C[kTC], S[kTC]
     static constexpr size_t st_off = cs_off + sizeof(long long) * 2 * kTC;               // int seg / raw start
-    static constexpr size_t comp_off = (st_off + sizeof(int) * 2 * kTC + 15) & ~(size_t)15;  // float [2][KZ][256]
-    static constexpr size_t bytes(bool kahan) {
-        return comp_off + (kahan ? sizeof(float) * 2 * KZ * kBpThreads : 0);
+    static constexpr size_t comp_off = (st_off + sizeof(int) * 2 * kTC + 15) & ~(size_t)15;  // float2 [KZ][256]
+    static constexpr int kSum = 32;  // tilts per compensated add of 16-bit volumes
+    static constexpr size_t bytes(bool kahan, int T) {
+        return comp_off + (kahan && T > kSum ? sizeof(float2) * KZ * kBpThreads : 0);
     }
 };
 
-// Voxels per thread along z: 16 for FP32 volumes (80 registers, three CTAs per SM); 8 for
-// 16-bit volumes, whose per-chunk partial sums double the voxel registers.
+// 16 voxels per thread along z: 80 registers, three CTAs per SM.
 template <int VT>
 struct Bp2Occ {
     static constexpr int value = 3;
-    static constexpr int kz = VT == kVolF32 ? 16 : 8;
+    static constexpr int kz = 16;
 };
 
 template <bool SANITIZE, bool POS, int VT, int KZ>
@@ -421,7 +427,7 @@ __device__ __forceinline__ void bp2_body(const BpLaunch& a, const int x0, const 
     long long* sS = sC + kTC;
     int* seg_start = reinterpret_cast<int*>(bsm + L::st_off);
     int* raw_start = seg_start + kTC;
-    float* comp_sh = reinterpret_cast<float*>(bsm + L::comp_off);
+    float2* parked = reinterpret_cast<float2*>(bsm + L::comp_off) + threadIdx.x;  // [KZ] by kBpThreads
 
     const int tid = threadIdx.x;
     const int tx = tid % kTX;
@@ -446,33 +452,26 @@ __device__ __forceinline__ void bp2_body(const BpLaunch& a, const int x0, const 
         vsc[0] = rin[0] ? a.vscale[r0] : 1.0f;
         vsc[1] = rin[1] ? a.vscale[r0 + 1] : 1.0f;
     }
-    float2 vx[KZ], pt[KZ];
-    {
-        const size_t v0 = ((size_t)zs * H + r0) * W + x;  // voxel (x, r0, zs); row r0 + 1 is W further
-        if (VT == kVolF32) {
-            const float* vb = static_cast<const float*>(a.vol) + v0;
-#pragma unroll
-            for (int k = 0; k < KZ; k++) {
-                vx[k].x = (k < nk && rin[0]) ? vb[k * plane] : 0.0f;
-                vx[k].y = (k < nk && rin[1]) ? vb[k * plane + W] : 0.0f;
-            }
-        } else {
-            const uint16_t* vb = static_cast<const uint16_t*>(a.vol) + v0;
-#pragma unroll
-            for (int k = 0; k < KZ; k++) {
-                vx[k].x = (k < nk && rin[0]) ? vol_load16<VT>(vb[k * plane]) * vsc[0] : 0.0f;
-                vx[k].y = (k < nk && rin[1]) ? vol_load16<VT>(vb[k * plane + W]) * vsc[1] : 0.0f;
-            }
-        }
+    float2 vx[KZ];  // the voxels; 16-bit volumes: the sum since the last compensated add
+    if (VT == kVolF32) {
+        // voxel (x, r0, zs); row r0 + 1 is W further
+        const float* vb = static_cast<const float*>(a.vol) + ((size_t)zs * H + r0) * W + x;
 #pragma unroll
         for (int k = 0; k < KZ; k++) {
-            pt[k] = make_float2(0.0f, 0.0f);
-            if (CHUNK_KAHAN) {
-                comp_sh[(0 * KZ + k) * kBpThreads + tid] = 0.0f;
-                comp_sh[(1 * KZ + k) * kBpThreads + tid] = 0.0f;
-            }
+            vx[k].x = (k < nk && rin[0]) ? vb[k * plane] : 0.0f;
+            vx[k].y = (k < nk && rin[1]) ? vb[k * plane + W] : 0.0f;
         }
+    } else {
+#pragma unroll
+        for (int k = 0; k < KZ; k++) vx[k] = make_float2(0.0f, 0.0f);
     }
+    // v + part with the compensation c (bp_add_kahan's steps, both rows)
+    auto kahan = [](float2& v, float2& c, float2 part) {
+        const float yx = part.x - c.x, yy = part.y - c.y;
+        const float tx_ = v.x + yx, ty_ = v.y + yy;
+        c = make_float2((tx_ - v.x) - yx, (ty_ - v.y) - yy);
+        v = make_float2(tx_, ty_);
+    };
 
     const int xa = x0, xb = min(x0 + kTX - 1, W - 1);
     const int za = z0, zb = min(z0 + L::kTZ2 - 1, D - 1);
@@ -559,9 +558,7 @@ __device__ __forceinline__ void bp2_body(const BpLaunch& a, const int x0, const 
             const int cnt = (int)((uint32_t)zi >> 16);
             const bool full = nk > 0 && kl <= 0 && kl + cnt >= KZ;
             auto add = [&](int k, float2 sv) {
-                if (CHUNK_KAHAN) {
-                    pt[k] = __fadd2_rn(pt[k], sv);
-                } else if (!SANITIZE && !POS) {
+                if (!SANITIZE && !POS) {
                     vx[k] = __fadd2_rn(vx[k], sv);
                 } else {
                     float cdummy = 0.0f;
@@ -594,58 +591,71 @@ __device__ __forceinline__ void bp2_body(const BpLaunch& a, const int x0, const 
                 }
             }
         }
-        if (CHUNK_KAHAN) {
+        if (CHUNK_KAHAN && (c0 + kTC) % L::kSum == 0 && c0 + kTC < a.T) {
+            // the first of two sums is complete
 #pragma unroll
             for (int k = 0; k < KZ; k++) {
-#pragma unroll
-                for (int q = 0; q < 2; q++) {
-                    float& vq = q ? vx[k].y : vx[k].x;
-                    const float part = q ? pt[k].y : pt[k].x;
-                    float cp = comp_sh[(q * KZ + k) * kBpThreads + tid];
-                    const float y = part - cp;
-                    const float tt = vq + y;
-                    cp = (tt - vq) - y;
-                    vq = tt;
-                    comp_sh[(q * KZ + k) * kBpThreads + tid] = cp;
-                }
-                pt[k] = make_float2(0.0f, 0.0f);
+                parked[k * kBpThreads] = vx[k];
+                vx[k] = make_float2(0.0f, 0.0f);
             }
         }
         __syncthreads();
     }
 
+    if (VT == kVolF32) {
 #pragma unroll
-    for (int q = 0; q < 2; q++) {
-        if (!rin[q]) continue;
-        const size_t v0 = ((size_t)zs * H + r0 + q) * W + x;
-        if (VT == kVolF32) {
-            float* vb = static_cast<float*>(a.vol) + v0;
+        for (int q = 0; q < 2; q++) {
+            if (!rin[q]) continue;
+            float* vb = static_cast<float*>(a.vol) + ((size_t)zs * H + r0 + q) * W + x;
 #pragma unroll
             for (int k = 0; k < KZ; k++)
                 if (k < nk) vb[k * plane] = q ? vx[k].y : vx[k].x;
-        } else {
-            uint16_t* vb = static_cast<uint16_t*>(a.vol) + v0;
-            const float inv = 1.0f / vsc[q];
-            float m = 0.0f;
-            bool range = false;
+        }
+    } else {
+        // store value / scale (exact: power of two) and feed the row maxima for re-scaling
+        uint16_t* vb = static_cast<uint16_t*>(a.vol) + ((size_t)zs * H + r0) * W + x;
+        const float inv[2] = {1.0f / vsc[0], 1.0f / vsc[1]};
+        float m[2] = {0.0f, 0.0f};
+        bool range = false;
+        constexpr int VS = VT == kVolF32 ? kVolF16 : VT;
+        constexpr int kLoads = 4;  // planes read before any of them is written
+        uint32_t old[kLoads];
 #pragma unroll
-            for (int k = 0; k < KZ; k++) {
-                if (k < nk) {
-                    const float v = (q ? vx[k].y : vx[k].x) - comp_sh[(q * KZ + k) * kBpThreads + tid];
-                    m = fmaxf(m, fabsf(v));
-                    float qv = v * inv;
-                    if (VT == kVolF16 && fabsf(qv) > kF16Max && isfinite(qv)) {
-                        range = true;
-                        qv = copysignf(kF16Max, qv);
-                    }
-                    vb[k * plane] = vol_store16<VT>(qv);
+        for (int k = 0; k < KZ; k++) {
+            if (k % kLoads == 0) {
+#pragma unroll
+                for (int i = 0; i < kLoads; i++) {
+                    const uint32_t lo = (k + i < nk && rin[0]) ? vb[(k + i) * plane] : 0;
+                    const uint32_t hi = (k + i < nk && rin[1]) ? vb[(k + i) * plane + W] : 0;
+                    old[i] = lo | hi << 16;
                 }
             }
+            if (k >= nk) continue;
+            const uint32_t ov = old[k % kLoads];
+            float2 v = make_float2(vol_load16<VS>((uint16_t)ov) * vsc[0], vol_load16<VS>((uint16_t)(ov >> 16)) * vsc[1]);
+            float2 c = make_float2(0.0f, 0.0f);
+            if (a.T > L::kSum) kahan(v, c, parked[k * kBpThreads]);
+            kahan(v, c, vx[k]);
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-            if ((tid & 31) == 0 && m > 0.0f) atomicMax(a.vmax + r0 + q, __float_as_uint(m));
-            if (range) atomicOr(a.status, (int)kStatusRange);
+            for (int q = 0; q < 2; q++) {
+                if (!rin[q]) continue;
+                const float val = q ? v.y - c.y : v.x - c.x;
+                m[q] = fmaxf(m[q], fabsf(val));
+                float qv = val * inv[q];
+                if (VT == kVolF16 && fabsf(qv) > kF16Max && isfinite(qv)) {
+                    range = true;
+                    qv = copysignf(kF16Max, qv);
+                }
+                vb[k * plane + q * W] = vol_store16<VS>(qv);
+            }
         }
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) m[q] = fmaxf(m[q], __shfl_xor_sync(0xffffffffu, m[q], o));
+            if ((tid & 31) == 0 && m[q] > 0.0f) atomicMax(a.vmax + r0 + q, __float_as_uint(m[q]));
+        }
+        if (range) atomicOr(a.status, (int)kStatusRange);
     }
 }
 
@@ -703,18 +713,21 @@ __global__ void __launch_bounds__(kBpCtaThreads, BpOcc<VT>::value)
 
 template <bool SANITIZE, bool POS, int VT>
 cudaError_t bp2_attr_one() {
-    const int m = (int)Bp2<Bp2Occ<VT>::kz>::bytes(VT != kVolF32);
+    const int m = (int)Bp2<Bp2Occ<VT>::kz>::bytes(VT != kVolF32, 1 << 30);
     cudaError_t e = cudaFuncSetAttribute(bp2_kernel<SANITIZE, POS, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, m);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(bp2_kernel_persist<SANITIZE, POS, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, m);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(bp2_kernel_batch<SANITIZE, POS, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, m);
+    if constexpr (VT == kVolF32) {
+        if (e != cudaSuccess) return e;
+        e = cudaFuncSetAttribute(bp2_kernel_persist<SANITIZE, POS, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, m);
+        if (e != cudaSuccess) return e;
+        e = cudaFuncSetAttribute(bp2_kernel_batch<SANITIZE, POS, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, m);
+    }
+    return e;
 }
 
 // FP32 volumes: every rule combination; 16-bit volumes: the plain form only.
 template <int VT>
 void bp2_vt(bool sanitize, bool positivity, const BpLaunch& a, dim3 grid, cudaStream_t s) {
-    const size_t sm = Bp2<Bp2Occ<VT>::kz>::bytes(VT != kVolF32);
+    const size_t sm = Bp2<Bp2Occ<VT>::kz>::bytes(VT != kVolF32, a.T);
     if constexpr (VT == kVolF32) {
         if (sanitize) {
             if (positivity) bp2_kernel<true, true, VT><<<grid, kBpThreads, sm, s>>>(a);
@@ -730,40 +743,26 @@ void bp2_vt(bool sanitize, bool positivity, const BpLaunch& a, dim3 grid, cudaSt
     }
 }
 
-template <int VT>
-void bp2_batch_vt(bool sanitize, bool positivity, const BpLaunch* descs, const int4* items, int n, cudaStream_t s) {
-    const size_t sm = Bp2<Bp2Occ<VT>::kz>::bytes(VT != kVolF32);
-    if constexpr (VT == kVolF32) {
-        if (sanitize) {
-            if (positivity) bp2_kernel_batch<true, true, VT><<<n, kBpThreads, sm, s>>>(descs, items);
-            else bp2_kernel_batch<true, false, VT><<<n, kBpThreads, sm, s>>>(descs, items);
-        } else {
-            if (positivity) bp2_kernel_batch<false, true, VT><<<n, kBpThreads, sm, s>>>(descs, items);
-            else bp2_kernel_batch<false, false, VT><<<n, kBpThreads, sm, s>>>(descs, items);
-        }
+void bp2_batch(bool sanitize, bool positivity, const BpLaunch* descs, const int4* items, int n, cudaStream_t s) {
+    const size_t sm = Bp2<Bp2Occ<kVolF32>::kz>::bytes(false, 0);
+    if (sanitize) {
+        if (positivity) bp2_kernel_batch<true, true, kVolF32><<<n, kBpThreads, sm, s>>>(descs, items);
+        else bp2_kernel_batch<true, false, kVolF32><<<n, kBpThreads, sm, s>>>(descs, items);
     } else {
-        (void)sanitize;
-        (void)positivity;
-        bp2_kernel_batch<false, false, VT><<<n, kBpThreads, sm, s>>>(descs, items);
+        if (positivity) bp2_kernel_batch<false, true, kVolF32><<<n, kBpThreads, sm, s>>>(descs, items);
+        else bp2_kernel_batch<false, false, kVolF32><<<n, kBpThreads, sm, s>>>(descs, items);
     }
 }
 
-template <int VT>
-void bp2_persist_vt(bool sanitize, bool positivity, const BpLaunch* descs, const int4* items, int n, int* cursor,
-                    int grid, cudaStream_t s) {
-    const size_t sm = Bp2<Bp2Occ<VT>::kz>::bytes(VT != kVolF32);
-    if constexpr (VT == kVolF32) {
-        if (sanitize) {
-            if (positivity) bp2_kernel_persist<true, true, VT><<<grid, kBpThreads, sm, s>>>(descs, items, n, cursor);
-            else bp2_kernel_persist<true, false, VT><<<grid, kBpThreads, sm, s>>>(descs, items, n, cursor);
-        } else {
-            if (positivity) bp2_kernel_persist<false, true, VT><<<grid, kBpThreads, sm, s>>>(descs, items, n, cursor);
-            else bp2_kernel_persist<false, false, VT><<<grid, kBpThreads, sm, s>>>(descs, items, n, cursor);
-        }
+void bp2_persist(bool sanitize, bool positivity, const BpLaunch* descs, const int4* items, int n, int* cursor, int grid,
+                 cudaStream_t s) {
+    const size_t sm = Bp2<Bp2Occ<kVolF32>::kz>::bytes(false, 0);
+    if (sanitize) {
+        if (positivity) bp2_kernel_persist<true, true, kVolF32><<<grid, kBpThreads, sm, s>>>(descs, items, n, cursor);
+        else bp2_kernel_persist<true, false, kVolF32><<<grid, kBpThreads, sm, s>>>(descs, items, n, cursor);
     } else {
-        (void)sanitize;
-        (void)positivity;
-        bp2_kernel_persist<false, false, VT><<<grid, kBpThreads, sm, s>>>(descs, items, n, cursor);
+        if (positivity) bp2_kernel_persist<false, true, kVolF32><<<grid, kBpThreads, sm, s>>>(descs, items, n, cursor);
+        else bp2_kernel_persist<false, false, kVolF32><<<grid, kBpThreads, sm, s>>>(descs, items, n, cursor);
     }
 }
 
@@ -807,8 +806,7 @@ int bp_tile_x() { return kTX; }
 int bp_tile_z() { return kTZ; }
 int bp_segment_pairs(bool wide) { return wide ? 192 : 96; }
 
-// FP32 volumes only: the 16-bit form's per-chunk partial sums cost more than the pairing
-// saves (measured: 89.9 against 85.7 ms per 2048 x 512 x 2048 x 121-tilt backprojection).
+// Batched forms pair the rows of FP32 volumes.
 bool bp_row_pairs(int vtype, bool sanitize, bool positivity) {
     (void)sanitize;
     (void)positivity;
@@ -831,10 +829,7 @@ cudaError_t launch_bp_batch(bool sanitize, bool positivity, int vtype, bool pair
     if (n_items <= 0) return cudaSuccess;
     if (pairs) {
         if (!bp_row_pairs(vtype, sanitize, positivity)) return cudaErrorInvalidValue;
-        if (vtype == kVolF32) bp2_batch_vt<kVolF32>(sanitize, positivity, descs, items, n_items, s);
-        else if (vtype == kVolBF16) bp2_batch_vt<kVolBF16>(sanitize, positivity, descs, items, n_items, s);
-        else if (vtype == kVolF16) bp2_batch_vt<kVolF16>(sanitize, positivity, descs, items, n_items, s);
-        else return cudaErrorInvalidValue;
+        bp2_batch(sanitize, positivity, descs, items, n_items, s);
         count_launch();
         return cudaGetLastError();
     }
@@ -847,7 +842,7 @@ cudaError_t launch_bp_batch(bool sanitize, bool positivity, int vtype, bool pair
 }
 
 int bp_persist_ctas_per_sm(int vtype, bool pairs) {
-    if (pairs) return vtype == kVolF32 ? Bp2Occ<kVolF32>::value : Bp2Occ<kVolF16>::value;
+    if (pairs) return Bp2Occ<kVolF32>::value;
     return vtype == kVolF32 ? BpOcc<kVolF32>::value : BpOcc<kVolF16>::value;
 }
 
@@ -856,10 +851,7 @@ cudaError_t launch_bp_persist(bool sanitize, bool positivity, int vtype, bool pa
     if (n_items <= 0) return cudaSuccess;
     if (pairs) {
         if (!bp_row_pairs(vtype, sanitize, positivity)) return cudaErrorInvalidValue;
-        if (vtype == kVolF32) bp2_persist_vt<kVolF32>(sanitize, positivity, descs, items, n_items, cursor, grid, s);
-        else if (vtype == kVolBF16) bp2_persist_vt<kVolBF16>(sanitize, positivity, descs, items, n_items, cursor, grid, s);
-        else if (vtype == kVolF16) bp2_persist_vt<kVolF16>(sanitize, positivity, descs, items, n_items, cursor, grid, s);
-        else return cudaErrorInvalidValue;
+        bp2_persist(sanitize, positivity, descs, items, n_items, cursor, grid, s);
     } else {
         if (vtype == kVolF32) bp_persist_vt<kVolF32>(sanitize, positivity, descs, items, n_items, cursor, grid, s);
         else if (vtype == kVolBF16) bp_persist_vt<kVolBF16>(sanitize, positivity, descs, items, n_items, cursor, grid, s);
@@ -878,7 +870,8 @@ cudaError_t launch_bp_separable(const BpLaunch& a, cudaStream_t s) {
     // fuller grid is faster (256 x 64 x 256: 0.093 against 0.126 ms)
     const long long ctas2 = (long long)g2.x * g2.y * g2.z;
     const bool big = ctas2 >= 2LL * Bp2Occ<kVolF32>::value * (a.sms > 0 ? a.sms : 148);
-    if (!a.bprow && !a.wide_seg && bp_row_pairs(a.vtype, a.sanitize, a.positivity) &&
+    const bool pairs = a.vtype == kVolF32 || (!a.sanitize && !a.positivity && a.T <= 2 * Bp2<16>::kSum);
+    if (!a.bprow && !a.wide_seg && pairs &&
         (a.rows_mode == 2 || (a.rows_mode == 0 && big))) {
         if (a.vtype == kVolF32) bp2_vt<kVolF32>(a.sanitize, a.positivity, a, g2, s);
         else if (a.vtype == kVolBF16) bp2_vt<kVolBF16>(false, false, a, g2, s);
