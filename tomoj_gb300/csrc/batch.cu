@@ -281,7 +281,8 @@ tomo_status build_plan(tomo_batch* b) {
                                 }
                     auto& fin = fpri[std::make_tuple(s, c, 0, 0)];
                     for (int t = 0; t < q.T; t++)
-                        for (int j = j0; j < g.h; j++) fin.push_back(make_int4(di, t, j, 0));
+                        for (int j = j0; j < g.h; j += kFinishRows)
+                            fin.push_back(make_int4(di, t, j, std::min(kFinishRows, g.h - j)));
                 }
             } else {
                 const int di = (int)fp.size();

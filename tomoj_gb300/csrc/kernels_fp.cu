@@ -167,90 +167,149 @@ __device__ __forceinline__ void add2(F2& s, float p, float pe) {
     s.hi = t;
 }
 
-// Projection, norm, difference and residual of one projection row from its segment sums
-// (the epilogue of fp_body with the sums read back, in segment order).  The squared
-// differences are summed in FP32 pairs with error terms, a warp's sums in FP64.  Bound by its
-// memory traffic (segment sums, ray table, measured row in; projection, norm and difference
-// out): 11 us for 7 tilts of 512 x 256 in 5 segments, where a form with seven FP64 operations
-// per ray took 27 us.
-__device__ __forceinline__ void finish_row(const FpLaunch& a, int b, int j) {
-    __shared__ double red[kFinishThreads / 32];
+// Projection, norm, difference and residual of n <= RJ consecutive projection rows from their
+// segment sums (the epilogue of fp_body with the sums read back, in segment order).  The
+// squared differences are summed in FP32 pairs with error terms, a warp's sums in FP64; a
+// row's order of adds depends on neither RJ nor UC.  Bound by its memory traffic (segment
+// sums, measured row in; projection, norm and difference out) when RJ rows share a ray's
+// 32-byte table entry, and by latency on grids of few rows, where UC columns of a row are
+// read at once instead.  One row and one column at a time took 13 us for 7 tilts of 512 x 256
+// in 5 segments, 482 us for 61 of 1024 x 1024 and 339 us for 12 series of 61 x 512 x 64;
+// these forms take 12, 374 and 284 us (two rows: 394 and 299 us for the last two).
+template <int RJ, int UC>
+__device__ __forceinline__ void finish_rows(const FpLaunch& a, int b, int j0, int n) {
+    __shared__ double red[RJ][kFinishThreads / 32];
     const int tilt = a.tilts[b];
-    const int r = a.two_rows ? a.rowmap[j] : j - a.row_off;
-    const bool row_in = r >= 0 && r < a.H;
-    // reduced storage: ray sums are in units of the row's slab scale (a power of two)
-    const float vsc = (a.vscale != nullptr && row_in) ? a.vscale[r] : 1.0f;
     const F2 ninc{a.ftilt[tilt].ninc_hi, a.ftilt[tilt].ninc_lo}, fac{a.factor_hi, a.factor_lo};
-    const size_t seg_stride = (size_t)a.T * a.h * a.w, row = ((size_t)b * a.h + j) * a.w;
+    const size_t seg_stride = (size_t)a.T * a.h * a.w, row = ((size_t)b * a.h + j0) * a.w;
     const float inv_seg = 1.0f / (float)a.rv.seg;
-    F2 e2{0.0f, 0.0f};
-    double far = 0.0;  // squares outside FP32's comfortable range
-    for (int i = threadIdx.x; i < a.w; i += kFinishThreads) {
-        const FpRay ray = a.rays[(size_t)tilt * a.w + i];
-        const float e = a.meas != nullptr ? a.meas[((size_t)tilt * a.h + j) * a.w + i] : 0.0f;
-        const int za = ray.zab & 0xFFFF, cnt = (int)((uint32_t)ray.zab >> 16);
-        const size_t o = row + i;
-        float th = __int_as_float(0x7fc00000), nrm = 0.0f;
-        if (cnt != 0 && row_in) {
-            // floor(z / seg): z + 1/2 keeps the product clear of whole numbers (z < 2^16)
-            const int s0 = (int)((za + 0.5f) * inv_seg), s1 = (int)((za + cnt - 0.5f) * inv_seg);
-            float sum = 0.0f;
-            for (int s = s0; s <= s1; s += 4) {
-                float v[4];
+    bool row_in[RJ];
+    float vsc[RJ];
+    F2 e2[RJ];
+    double far[RJ];  // squares outside FP32's comfortable range
 #pragma unroll
-                for (int q = 0; q < 4; q++) v[q] = s + q <= s1 ? __ldcg(a.part + (s + q) * seg_stride + o) : 0.0f;
+    for (int y = 0; y < RJ; y++) {
+        const int r = y >= n ? -1 : a.two_rows ? a.rowmap[j0 + y] : j0 + y - a.row_off;
+        row_in[y] = r >= 0 && r < a.H;
+        // reduced storage: ray sums are in units of the row's slab scale (a power of two)
+        vsc[y] = (a.vscale != nullptr && row_in[y]) ? a.vscale[r] : 1.0f;
+        e2[y] = F2{0.0f, 0.0f};
+        far[y] = 0.0;
+    }
+    for (int i0 = threadIdx.x; i0 < a.w; i0 += kFinishThreads * UC) {
+        float e[UC][RJ], sum[UC][RJ], nrm[UC];
+        int s0[UC], s1[UC], smin = a.rv.nseg, smax = -1;
 #pragma unroll
-                for (int q = 0; q < 4; q++) sum += v[q];
-            }
-            th = mul_split(sum * vsc, ninc).hi;
-            nrm = ray.norm;
-        }
-        a.proj[o] = th;
-        a.norm[o] = nrm;
-        if (a.meas != nullptr) {
-            float d = 0.0f;
-            if (!isnan(e) && !isnan(th)) {
-                const F2 v = mul_split(__fdiv_rn(__fsub_rn(e, th), nrm), fac);
-                d = v.hi;
-                const float m = fabsf(d);
-                if ((m > 1e15f || m < 1e-15f) && d != 0.0f) {
-                    far += (double)d * d;
-                } else {
-                    const float p = d * d;
-                    add2(e2, p, fmaf(d, d, -p) + 2.0f * d * v.lo);
+        for (int c = 0; c < UC; c++) {
+            const int i = i0 + c * kFinishThreads;
+            s0[c] = a.rv.nseg;
+            s1[c] = -1;
+            nrm[c] = 0.0f;
+            if (i < a.w) {
+                const FpRay& ray = a.rays[(size_t)tilt * a.w + i];
+                const int zab = ray.zab, za = zab & 0xFFFF, cnt = (int)((uint32_t)zab >> 16);
+                nrm[c] = ray.norm;
+                if (cnt != 0) {
+                    // floor(z / seg): z + 1/2 keeps the product clear of whole numbers (z < 2^16)
+                    s0[c] = (int)((za + 0.5f) * inv_seg);
+                    s1[c] = (int)((za + cnt - 0.5f) * inv_seg);
                 }
             }
-            a.diff[o] = d;
+            smin = min(smin, s0[c]);
+            smax = max(smax, s1[c]);
+#pragma unroll
+            for (int y = 0; y < RJ; y++) {
+                e[c][y] = (a.meas != nullptr && y < n && i < a.w)
+                              ? a.meas[((size_t)tilt * a.h + j0 + y) * a.w + i] : 0.0f;
+                sum[c][y] = 0.0f;
+            }
+        }
+        for (int s = smin; s <= smax; s += 4) {
+            float v[4][UC][RJ];
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+#pragma unroll
+                for (int c = 0; c < UC; c++)
+#pragma unroll
+                    for (int y = 0; y < RJ; y++)
+                        v[q][c][y] = (s + q >= s0[c] && s + q <= s1[c] && row_in[y])
+                                         ? __ldcg(a.part + (s + q) * seg_stride + row + (size_t)y * a.w + i0 + c * kFinishThreads)
+                                         : 0.0f;
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+#pragma unroll
+                for (int c = 0; c < UC; c++)
+#pragma unroll
+                    for (int y = 0; y < RJ; y++) sum[c][y] += v[q][c][y];
+        }
+#pragma unroll
+        for (int c = 0; c < UC; c++) {
+            const int i = i0 + c * kFinishThreads;
+            if (i >= a.w) continue;
+#pragma unroll
+            for (int y = 0; y < RJ; y++) {
+                if (y >= n) continue;
+                const size_t o = row + (size_t)y * a.w + i;
+                float th = __int_as_float(0x7fc00000), nr = 0.0f;
+                if (s1[c] >= 0 && row_in[y]) {
+                    th = mul_split(sum[c][y] * vsc[y], ninc).hi;
+                    nr = nrm[c];
+                }
+                a.proj[o] = th;
+                a.norm[o] = nr;
+                if (a.meas != nullptr) {
+                    float d = 0.0f;
+                    if (!isnan(e[c][y]) && !isnan(th)) {
+                        const F2 v = mul_split(__fdiv_rn(__fsub_rn(e[c][y], th), nr), fac);
+                        d = v.hi;
+                        const float m = fabsf(d);
+                        if ((m > 1e15f || m < 1e-15f) && d != 0.0f) {
+                            far[y] += (double)d * d;
+                        } else {
+                            const float p = d * d;
+                            add2(e2[y], p, fmaf(d, d, -p) + 2.0f * d * v.lo);
+                        }
+                    }
+                    a.diff[o] = d;
+                }
+            }
         }
     }
     if (a.meas != nullptr) {
-        // the lanes' sums in fixed order, without FP64 (an infinite sum has no error term)
 #pragma unroll
-        for (int q = 16; q > 0; q >>= 1) {
-            const float oh = __shfl_down_sync(0xffffffffu, e2.hi, q), ol = __shfl_down_sync(0xffffffffu, e2.lo, q);
-            add2(e2, oh, ol);
+        for (int y = 0; y < RJ; y++) {
+            // the lanes' sums in fixed order, without FP64 (an infinite sum has no error term)
+#pragma unroll
+            for (int q = 16; q > 0; q >>= 1) {
+                const float oh = __shfl_down_sync(0xffffffffu, e2[y].hi, q);
+                const float ol = __shfl_down_sync(0xffffffffu, e2[y].lo, q);
+                add2(e2[y], oh, ol);
+            }
+            if (__any_sync(0xffffffffu, far[y] != 0.0)) far[y] = warp_sum(far[y]);
+            if ((threadIdx.x & 31) == 0)
+                red[y][threadIdx.x >> 5] =
+                    (isfinite(e2[y].hi) ? (double)e2[y].hi + (double)e2[y].lo : (double)e2[y].hi) + far[y];
         }
-        if (__any_sync(0xffffffffu, far != 0.0)) far = warp_sum(far);
-        if ((threadIdx.x & 31) == 0)
-            red[threadIdx.x >> 5] = (isfinite(e2.hi) ? (double)e2.hi + (double)e2.lo : (double)e2.hi) + far;
         __syncthreads();
-        if (threadIdx.x == 0) {
+        if (threadIdx.x < n) {
             double sum = 0.0;
-            for (int k = 0; k < kFinishThreads / 32; k++) sum += red[k];
-            a.errpart[(size_t)b * a.h + j] = sum;
+            for (int k = 0; k < kFinishThreads / 32; k++) sum += red[threadIdx.x][k];
+            a.errpart[(size_t)b * a.h + j0 + threadIdx.x] = sum;
         }
     }
 }
 
+template <int RJ, int UC>
 __global__ void __launch_bounds__(kFinishThreads) fp_finish_kernel(const __grid_constant__ FpLaunch a) {
-    finish_row(a, blockIdx.y, a.j0 + blockIdx.x);
+    const int j = a.j0 + blockIdx.x * RJ;
+    finish_rows<RJ, UC>(a, blockIdx.y, j, min(RJ, a.j1 - j));
 }
 
-// Batched form: block b runs items[b] = {problem, tilt, row, -}.
-__global__ void __launch_bounds__(kFinishThreads)
+// Batched form: block b runs items[b] = {problem, tilt, first row, rows}.
+__global__ void __launch_bounds__(kFinishThreads, 8)
     fp_finish_batch_kernel(const FpLaunch* __restrict__ descs, const int4* __restrict__ items) {
     const int4 it = items[blockIdx.x];
-    finish_row(descs[it.x], it.y, it.z);
+    finish_rows<kFinishRows, 1>(descs[it.x], it.y, it.z, it.w);
 }
 
 }  // namespace
@@ -396,7 +455,13 @@ cudaError_t launch_fpr(const FpLaunch& a0, cudaStream_t s) {
         if (e != cudaSuccess) return e;
         count_launch();
     }
-    fp_finish_kernel<<<dim3((unsigned)(a.j1 - a.j0), (unsigned)a.T), kFinishThreads, 0, s>>>(a);
+    // rows in groups where that still fills the resident blocks (16 per SM)
+    const long long rows = a.j1 - a.j0;
+    if (rows * a.T >= 16LL * kFinishRows * device_sms())
+        fp_finish_kernel<kFinishRows, 1><<<dim3((unsigned)((rows + kFinishRows - 1) / kFinishRows), (unsigned)a.T),
+                                           kFinishThreads, 0, s>>>(a);
+    else
+        fp_finish_kernel<1, 4><<<dim3((unsigned)rows, (unsigned)a.T), kFinishThreads, 0, s>>>(a);
     count_launch();
     return cudaGetLastError();
 }

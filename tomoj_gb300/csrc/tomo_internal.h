@@ -202,7 +202,9 @@ cudaError_t launch_fpr_batch(int zc, int eb, const FpLaunch* descs, const int4* 
 // (zero before the launch), whatever their chunk depth.
 cudaError_t launch_fpr_persist(const FpLaunch* descs, const int4* items, int n_items, int* cursor, int grid,
                                size_t smem, cudaStream_t s);
-// The closing pass of many problems: block b runs items[b] = {problem, tilt, row, -}.
+// The closing pass of many problems: block b runs items[b] = {problem, tilt, first row,
+// rows} of at most kFinishRows rows.
+constexpr int kFinishRows = 4;
 cudaError_t launch_fp_finish_batch(const FpLaunch* descs, const int4* items, int n, cudaStream_t s);
 // Any geometry (kernels_generic.cu): one thread per ray / voxel in the reference's
 // double arithmetic.  proj/norm are [T][h][w] in batch order.
