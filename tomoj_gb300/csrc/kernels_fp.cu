@@ -455,13 +455,18 @@ cudaError_t launch_fpr(const FpLaunch& a0, cudaStream_t s) {
         if (e != cudaSuccess) return e;
         count_launch();
     }
-    // rows in groups where that still fills the resident blocks (16 per SM)
+    // rows in groups where that still fills the resident blocks (16 per SM), else as many columns at
+    // once as a row has per thread
     const long long rows = a.j1 - a.j0;
     if (rows * a.T >= 16LL * kFinishRows * device_sms())
         fp_finish_kernel<kFinishRows, 1><<<dim3((unsigned)((rows + kFinishRows - 1) / kFinishRows), (unsigned)a.T),
                                            kFinishThreads, 0, s>>>(a);
-    else
+    else if (a.w > 2 * kFinishThreads)
         fp_finish_kernel<1, 4><<<dim3((unsigned)rows, (unsigned)a.T), kFinishThreads, 0, s>>>(a);
+    else if (a.w > kFinishThreads)
+        fp_finish_kernel<1, 2><<<dim3((unsigned)rows, (unsigned)a.T), kFinishThreads, 0, s>>>(a);
+    else
+        fp_finish_kernel<1, 1><<<dim3((unsigned)rows, (unsigned)a.T), kFinishThreads, 0, s>>>(a);
     count_launch();
     return cudaGetLastError();
 }
