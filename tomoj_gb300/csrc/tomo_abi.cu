@@ -154,10 +154,18 @@ void free_n(tomo_projector* p, T** ptr, size_t n) {
     *ptr = nullptr;
 }
 
-tomo_status check_status(tomo_projector* p) {
-    int st = 0;
-    CK(cudaMemcpyAsync(&st, p->d_status, sizeof(int), cudaMemcpyDeviceToHost, p->stream));
+// Waits for the handle's stream and reads the status word and, with err, the first T error sums in
+// the same copy (d_status lies in the double before d_err).
+tomo_status check_status(tomo_projector* p, double* err = nullptr, int T = 0) {
+    if (!err) T = 0;
+    p->h_errstat.resize(std::max<size_t>(p->h_errstat.size(), (size_t)T + 1));
+    CK(cudaMemcpyAsync(p->h_errstat.data(), p->d_status, sizeof(double) * ((size_t)T + 1), cudaMemcpyDeviceToHost,
+                       p->stream));
     CK(cudaStreamSynchronize(p->stream));
+    p->batch_in_flight = false;
+    int st = 0;
+    std::memcpy(&st, p->h_errstat.data(), sizeof(int));
+    if (T > 0) std::memcpy(err, p->h_errstat.data() + 1, sizeof(double) * T);
     if (st != 0) {
         CK(cudaMemsetAsync(p->d_status, 0, sizeof(int), p->stream));
         // a kernel that gave up may have left depth-split tickets behind
@@ -172,11 +180,14 @@ tomo_status check_status(tomo_projector* p) {
 
 tomo_status upload_batch(tomo_projector* p) {
     if (p->batch_uploaded) return TOMO_OK;
-    if (!p->batch.empty())
-        CK(cudaMemcpyAsync(p->d_batch, p->batch.data(), p->batch.size() * sizeof(int), cudaMemcpyHostToDevice,
+    if (!p->batch.empty()) {
+        // from a copy that stays as it is until the stream has been waited for
+        if (p->batch_in_flight) CK(cudaStreamSynchronize(p->stream));
+        p->h_batch = p->batch;
+        p->batch_in_flight = true;
+        CK(cudaMemcpyAsync(p->d_batch, p->h_batch.data(), p->h_batch.size() * sizeof(int), cudaMemcpyHostToDevice,
                            p->stream));
-    // the host vector may change after this call: make the copy complete first
-    CK(cudaStreamSynchronize(p->stream));
+    }
     p->batch_uploaded = true;
     return TOMO_OK;
 }
@@ -733,9 +744,8 @@ tomo_status tomo_create(const tomo_geom* geom, const tomo_params* params, tomo_p
     A(alloc_n(p, &p->d_diff, N * p->npix));
     A(alloc_n(p, &p->d_obatch, N * p->npix));
     A(alloc_n(p, &p->d_errpart, N * g.h));
-    A(alloc_n(p, &p->d_err, N));
+    A(alloc_n(p, &p->d_err, N + 1));
     A(alloc_n(p, &p->d_batch, N));
-    A(alloc_n(p, &p->d_status, 1));
     A(alloc_n(p, &p->d_flags, 1));
     A(alloc_n(p, &p->d_ftilt, N));
     A(alloc_n(p, &p->d_rays, N * g.w));
@@ -770,8 +780,9 @@ tomo_status tomo_create(const tomo_geom* geom, const tomo_params* params, tomo_p
     } else {
         launch_vol_fill(p->d_vol16, p->vtype, p->d_vscale, p->d_vmax, p->nvox, g.H, 0.0f, p->stream);
     }
-    cudaMemsetAsync(p->d_status, 0, sizeof(int), p->stream);
-    cudaMemsetAsync(p->d_err, 0, sizeof(double) * N, p->stream);
+    cudaMemsetAsync(p->d_err, 0, sizeof(double) * (N + 1), p->stream);
+    p->d_status = reinterpret_cast<int*>(p->d_err);
+    p->d_err++;
     if (cudaStreamSynchronize(p->stream) != cudaSuccess) {
         tomo_destroy(p);
         return fail(TOMO_ERR_CUDA, "initialisation failed");
@@ -1301,9 +1312,7 @@ tomo_status tomo_project_and_difference(tomo_projector* p, double factor, int32_
     CKS(upload_batch(p));
     const int T = (int)p->batch.size();
     CKS(run_fp(p, p->d_batch, T, y0, true, factor, 0));
-    if (err_out && T > 0)
-        CK(cudaMemcpyAsync(err_out, p->d_err, sizeof(double) * T, cudaMemcpyDeviceToHost, p->stream));
-    CKS(check_status(p));
+    CKS(check_status(p, err_out, T));
     p->projected = true;
     p->diffs_valid = true;
     return TOMO_OK;

@@ -35,7 +35,10 @@ struct tomo_projector {
     float* d_diff = nullptr;
     float* d_obatch = nullptr;
     double* d_errpart = nullptr;
-    double* d_err = nullptr;
+    double* d_err = nullptr;         // [N], after the double that holds d_status
+    std::vector<double> h_errstat;   // check_status's copy of both
+    std::vector<int> h_batch;        // upload_batch's source
+    bool batch_in_flight = false;    // its copy may still read h_batch
     int* d_batch = nullptr;
     int* d_orders = nullptr;
     int orders_cap = 0;
