@@ -247,8 +247,11 @@ int fp_split(tomo_projector* p, int T, int rows, int tpc) {
 
 // Row-vector form: its plan for T tilts and the tilts per launch (see handle_fpr_prepare).
 // The segment sums of a launch take at most eight times the series' size (the handle holds
-// six such buffers) and 1 GiB; more tilts run in further launches.  Volumes that hold NaN or Inf stay
-// on the one-row form, whose samples treat them as before.
+// six such buffers) and 1 GiB, or half the bytes of an FP32 volume where that is more (every launch
+// reads the volume again: a SIRT iteration of 2048 x 512 x 2048 with 121 tilts takes 176 ms in launches
+// of five tilts, 161 ms in launches of 24); more tilts run in further launches.  Memory that is
+// refused leaves the 1 GiB, then the one-row form.  Volumes that hold NaN or Inf stay on the
+// one-row form, whose samples treat them as before.
 int fpr_prepare(tomo_projector* p, int T, FprPlan* plan) {
     const Geometry& g = p->g;
     if (T <= 0 || !g.separable || p->vol_flag()) return 0;
@@ -265,9 +268,14 @@ int fpr_prepare(tomo_projector* p, int T, FprPlan* plan) {
     *plan = *have;
     if (plan->zc == 0) return 0;
     const size_t per_tilt = (size_t)plan->nseg * p->npix;
-    const size_t lim = std::min<size_t>((size_t)8 * g.N * p->npix, (size_t)1 << 28);
-    int tc = (int)std::min<size_t>((size_t)T, std::max<size_t>(1, lim / per_tilt));
-    if (tc < T && tc >= plan->tg) tc -= tc % plan->tg;
+    const size_t base = (size_t)1 << 28;
+    auto tilts = [&](size_t room) {
+        const size_t lim = std::min<size_t>((size_t)8 * g.N * p->npix, room);
+        int tc = (int)std::min<size_t>((size_t)T, std::max<size_t>(1, lim / per_tilt));
+        if (tc < T && tc >= plan->tg) tc -= tc % plan->tg;
+        return tc;
+    };
+    int tc = tilts(p->fpr_denied ? base : std::max(base, p->nvox / 2));
     if (p->tilts_per_cta > 0) plan->tg = std::min({p->tilts_per_cta, kFprMaxTilts, T});
     const size_t need = per_tilt * (size_t)tc;
     if (need > p->fppart_cap) {
@@ -275,8 +283,14 @@ int fpr_prepare(tomo_projector* p, int T, FprPlan* plan) {
         if (cudaStreamIsCapturing(p->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return 0;
         free_n(p, &p->d_fppart, p->fppart_cap);
         p->fppart_cap = 0;
-        if (alloc_n(p, &p->d_fppart, need) != TOMO_OK) return 0;
-        p->fppart_cap = need;
+        size_t got = need;
+        if (alloc_n(p, &p->d_fppart, got) != TOMO_OK) {
+            p->fpr_denied = true;
+            tc = tilts(base);
+            got = per_tilt * (size_t)tc;
+            if (got >= need || alloc_n(p, &p->d_fppart, got) != TOMO_OK) return 0;
+        }
+        p->fppart_cap = got;
     }
     return tc;
 }

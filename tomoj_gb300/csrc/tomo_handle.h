@@ -135,6 +135,7 @@ struct tomo_projector {
     // forward-projector depth split scratch (partial ray sums, per-group tickets)
     float* d_fppart = nullptr;
     size_t fppart_cap = 0;  // floats
+    bool fpr_denied = false;  // the larger scratch of the row-vector projector was refused
     unsigned* d_tickets = nullptr;
     size_t tickets_cap = 0;
     // per-kernel timing of the OS-SART driver (tomo_set_profiling)
