@@ -1,6 +1,7 @@
-// Forward-projection dispatch: picks the kernel instantiation for the number of
-// detector columns each thread owns (QP = ceil(w / threads)); the kernel itself is in
-// fp_kernel.cuh and is compiled once per (threads, QP) pair (fp_kernel_q*.cu).
+// Forward-projection dispatch: the row-vector form's plan, launches and closing pass
+// (kernel in fpr_kernel.cuh, compiled once per chunk depth in fpr_kernel_z*.cu), and the
+// one-row form's instantiation for the number of detector columns each thread owns
+// (QP = ceil(w / threads); kernel in fp_kernel.cuh, one per (threads, QP) in fp_kernel_q*.cu).
 #include <algorithm>
 #include <cmath>
 #include <functional>
