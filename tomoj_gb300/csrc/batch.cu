@@ -10,8 +10,8 @@
 // (tomo_batch_set_persistent) the forward launches of a phase are one persistent launch
 // instead: resident CTAs take items from a list, longest first, through an
 // atomic cursor, and the launches of a phase run side by side.  The
-// per-member descriptors and work lists are rebuilt only when the membership
-// or the update sizes change, and the step's launches are captured once as a
+// per-member descriptors and work lists are rebuilt only when the membership,
+// the update sizes or a member's state (series, geometry, options, scratch) change, and the step's launches are captured once as a
 // CUDA graph and replayed while they stay valid; every iteration only uploads
 // the members' new orderings (orderShuffleART with the given first index) and
 // reads their residuals back.
@@ -107,7 +107,7 @@ struct tomo_batch {
     std::vector<BpSeg> bp_segs;
     std::vector<RedSeg> red_segs;
     std::vector<FprSeg> fpr_segs;
-    std::vector<const float*> parts;  // members' segment-sum scratch the plan was built on
+    std::vector<std::pair<uint64_t, bool>> states;  // handle_plan_state of the members the plan was built on
     std::vector<BpPSeg> bp_psegs;
     int persistent = 0;  // tomo_batch_set_persistent mode (default: a launch per kernel variant)
     int* d_cursor = nullptr;
@@ -186,7 +186,8 @@ tomo_status build_plan(tomo_batch* b) {
     std::map<std::tuple<int, int, int, int>, std::vector<int4>> fpri;
     std::map<std::tuple<int, int, int, int>, std::vector<double>> fprcost;
     std::map<std::tuple<int, int, int, int>, size_t> fprsmem;
-    b->parts.clear();
+    b->plan_valid = false;  // until this one is complete
+    b->states.clear();
     std::map<int, std::vector<ErrReduce>> reds;
     std::map<int, std::vector<VolJob>> vjobs;
     b->max_nsub = 0;
@@ -209,7 +210,7 @@ tomo_status build_plan(tomo_batch* b) {
             FprPlan plan{};
             handle_fpr_prepare(p, T, &plan);
         }
-        b->parts.push_back(p->d_fppart);
+        b->states.push_back(handle_plan_state(p));
         // rows the forward projector never writes must read as zero residual
         BCK(cudaMemsetAsync(p->d_errpart, 0, sizeof(double) * (size_t)N * g.h, b->stream));
         const int qp = fp_qp(g.w), nt = fp_threads(g.w);
@@ -612,8 +613,8 @@ tomo_status tomo_batch_iteration(tomo_batch* b, const double* relax, const int32
         upd[m] = update[m] == 0 ? N : std::min(update[m], N);
         fac[m] = (double)(float)(relax[m] / upd[m]);  // float factorimg (TomoReconstruction2.java:646)
     }
-    // a member's own calls may have moved its segment-sum scratch
-    for (size_t m = 0; b->plan_valid && m < M; m++) b->plan_valid = b->parts[m] == b->members[m]->d_fppart;
+    // a member's own calls may have changed what the plan and its graph were made of
+    for (size_t m = 0; b->plan_valid && m < M; m++) b->plan_valid = b->states[m] == handle_plan_state(b->members[m]);
     if (!b->plan_valid || upd != b->upd || fac != b->factor) {
         b->upd = upd;
         b->factor = fac;

@@ -232,6 +232,7 @@ int fp_split(tomo_projector* p, int T, int rows, int tpc) {
     if (need_part > p->fppart_cap) {
         free_n(p, &p->d_fppart, p->fppart_cap);
         p->fppart_cap = 0;
+        p->plan_gen++;
         if (alloc_n(p, &p->d_fppart, need_part) != TOMO_OK) return 1;
         p->fppart_cap = need_part;
     }
@@ -283,6 +284,7 @@ int fpr_prepare(tomo_projector* p, int T, FprPlan* plan) {
         if (cudaStreamIsCapturing(p->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return 0;
         free_n(p, &p->d_fppart, p->fppart_cap);
         p->fppart_cap = 0;
+        p->plan_gen++;
         size_t got = need;
         if (alloc_n(p, &p->d_fppart, got) != TOMO_OK) {
             p->fpr_denied = true;
@@ -883,6 +885,7 @@ tomo_status tomo_set_stream(tomo_projector* p, void* stream) {
 static tomo_status setup_geometry(tomo_projector* p) {
     Geometry& g = p->g;
     const int N = g.N;
+    p->plan_gen++;
     bool integral = true, vertical = true;
     for (int t = 0; t < N; t++) {
         integral = integral && tilt_is_separable(&p->euler[9 * t], g);
@@ -1037,6 +1040,7 @@ tomo_status tomo_load_series(tomo_projector* p, const float* pixels, int32_t pix
     p->meas_has_nan = (flags & 1) != 0;
     p->meas_has_inf = (flags & 2) != 0;
     p->meas_filled = (flags & 4) != 0;
+    p->plan_gen++;
     p->series_loaded = true;
     p->batch.clear();
     p->batch_uploaded = false;
@@ -1058,6 +1062,7 @@ tomo_status tomo_set_row_streams(tomo_projector* p, int32_t k) {
 tomo_status tomo_set_positivity(tomo_projector* p, int32_t enabled) {
     if (!p) return fail(TOMO_ERR_INVALID, "null handle");
     p->params.positivity = enabled ? 1 : 0;
+    p->plan_gen++;
     return TOMO_OK;
 }
 
@@ -1128,6 +1133,7 @@ tomo_status tomo_set_fill(tomo_projector* p, int32_t fill) {
     p->meas_has_nan = (flags & 1) != 0;
     p->meas_has_inf = (flags & 2) != 0;
     p->meas_filled = (flags & 4) != 0;
+    p->plan_gen++;
     p->obatch_valid = false;
     return TOMO_OK;
 }
@@ -1268,6 +1274,7 @@ tomo_status tomo_share_volume(tomo_projector* p, tomo_projector* owner) {
         p->d_vol = mine;
         p->vol_owner = nullptr;
         p->stream = p->own_stream;
+        p->plan_gen++;
         return TOMO_OK;
     }
     if (owner->vol_owner) return fail(TOMO_ERR_INVALID, "the owner shares another handle's volume");
@@ -1281,6 +1288,7 @@ tomo_status tomo_share_volume(tomo_projector* p, tomo_projector* owner) {
     if (!p->vol_owner) free_n(p, &p->d_vol, p->nvox);
     p->d_vol = owner->d_vol;
     p->vol_owner = owner;
+    p->plan_gen++;
     p->stream = owner->stream;
     owner->vol_sharers.push_back(p);
     return TOMO_OK;
@@ -1528,6 +1536,7 @@ tomo_status tomo_set_tvm(tomo_projector* p, float theta, float g, float dt, int3
     p->tv_g = g;
     p->tv_dt = dt;
     p->tv_iters = iterations;
+    p->plan_gen++;
     return TOMO_OK;
 }
 
@@ -1538,6 +1547,7 @@ tomo_status tomo_set_fista(tomo_projector* p, int32_t enabled) {
     if (enabled && !p->d_prev) CKS(alloc_n(p, &p->d_prev, p->nvox));
     p->fista = enabled != 0;
     p->fista_t = 0.0;
+    p->plan_gen++;
     return TOMO_OK;
 }
 
@@ -1549,6 +1559,7 @@ tomo_status tomo_set_bayesian(tomo_projector* p, double lambda, double alpha, in
     p->bayes = enabled != 0;
     p->bayes_lambda = lambda;
     p->bayes_alpha = alpha;
+    p->plan_gen++;
     return TOMO_OK;
 }
 
@@ -1564,6 +1575,7 @@ tomo_status tomo_set_bgart(tomo_projector* p, double k, int32_t dark_bg, int32_t
     p->bg_dark = dark_bg != 0;
     p->bg_median = do_median != 0;
     p->bg_value = bg_value;
+    p->plan_gen++;
     if (p->bgart) {
         // the reference's constructor collapses the starting volume once (BgARTVoxelProjector3D.java:22-27)
         CK(launch_bgart_collapse(p->d_vol, p->nvox, k, p->bg_dark, bg_value, p->d_bgscratch, p->stream));
@@ -1575,6 +1587,7 @@ tomo_status tomo_set_bgart(tomo_projector* p, double k, int32_t dark_bg, int32_t
 tomo_status tomo_set_compressed_sensing(tomo_projector* p, int32_t wavelet_type, double degree, double shift,
                                        double fraction_zeros, const int32_t* levels, int32_t enabled) {
     if (!p) return fail(TOMO_ERR_INVALID, "null handle");
+    p->plan_gen++;
     if (!enabled) {
         p->cs = false;
         return TOMO_OK;
@@ -1650,6 +1663,7 @@ tomo_status tomo_profile_read(tomo_projector* p, double* out4) {
 tomo_status tomo_set_bp_rows(tomo_projector* p, int32_t rows) {
     if (!p || rows < 0 || rows > 2) return fail(TOMO_ERR_INVALID, "rows per backprojection thread: 0, 1 or 2");
     p->bp_rows = rows;
+    p->plan_gen++;
     return TOMO_OK;
 }
 
@@ -1735,6 +1749,7 @@ tomo_status tomo_autotune(tomo_projector* p, int32_t update, int32_t reps, doubl
             }
         }
         p->bp_rows = best_r;
+        p->plan_gen++;
         ck(cudaMemcpyAsync(p->vol(), save, vbytes, cudaMemcpyDeviceToDevice, p->stream));
         if (save_sc) ck(cudaMemcpyAsync(p->d_vscale, save_sc, sizeof(float) * g.H, cudaMemcpyDeviceToDevice, p->stream));
         if (save_mx)
@@ -1760,6 +1775,7 @@ tomo_status tomo_autotune(tomo_projector* p, int32_t update, int32_t reps, doubl
 tomo_status tomo_set_tilts_per_cta(tomo_projector* p, int32_t n) {
     if (!p || n < 0) return fail(TOMO_ERR_INVALID, "bad argument");
     p->tilts_per_cta = n;
+    p->plan_gen++;
     return TOMO_OK;
 }
 

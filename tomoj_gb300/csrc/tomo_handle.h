@@ -1,6 +1,7 @@
 // The projector handle (shared by the C-ABI translation units).
 #pragma once
 #include <atomic>
+#include <utility>
 #include <vector>
 
 #include "../../include/tomoj_gb300.h"
@@ -119,6 +120,9 @@ struct tomo_projector {
     // volume a backprojection of differences adds to
     void* bp_target() const { return bayes ? static_cast<void*>(d_dist) : vol(); }
     std::atomic<int> cancel{0};
+    // raised by every call that changes what a batch's plan and graph are made of: geometry
+    // tables and the cuts that depend on them, series flags, options, kernel shapes, buffers
+    uint64_t plan_gen = 0;
     int tilts_per_cta = 0;  // forward projector tilt grouping (0 = automatic)
     int bp_rows = 0;        // backprojection rows per thread (0 = automatic, 1, 2)
     int hold_first_copy = 0;  // failure-path test hook of the forward projector (tomo_debug_hold_first_copy)
@@ -155,6 +159,10 @@ tomo_status handle_fail(tomo_status code, const char* msg);
 tomo_status handle_need_series(tomo_projector* p);
 tomo_status handle_start_iteration(tomo_projector* p);
 tomo_status handle_end_iteration(tomo_projector* p);
+// What a batch's plan of this handle depends on besides the update: a value that changes with
+// it (handle calls that change it, and the non-finite flag of the volume, which a handle
+// sharing the volume may set too).
+inline std::pair<uint64_t, bool> handle_plan_state(tomo_projector* p) { return {p->plan_gen, p->vol_flag()}; }
 int handle_tilts_per_cta(const tomo_projector* p, int T);
 // Plan of the row-vector forward projector for updates of T tilts and the tilts one launch
 // takes (the partial sums' scratch is bounded); 0: the handle's projections run the one-row
