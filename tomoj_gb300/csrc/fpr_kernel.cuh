@@ -48,7 +48,8 @@ constexpr int kRays = 32;                     // rays per block (one per lane)
 constexpr int kMaxNB = 4096 / kRays;          // ray blocks of a detector row (w <= 4096)
 constexpr uint32_t kWaitTries = 1u << 24;
 
-// Shared memory: barrier | per-slot info | block lists | two plane buffers.
+// Shared memory: barrier | a column of zeros | per-slot info | block lists | two plane buffers.
+constexpr int kZeroOff = 32;                                    // float [8]
 constexpr int kInfoOff = 64;                                    // BlockInfo [kCap]
 constexpr int kZabOff = kInfoOff + kCap * 32;                   // int [kCap][32] plane intervals
 constexpr int kStepOff = kZabOff + kCap * 128;                  // long long [kFprMaxTilts]
@@ -186,18 +187,17 @@ __device__ __noinline__ Rows8 partial_chunk(unsigned buf, int pitch, Chunk c, lo
 #pragma unroll
     for (int zz = 0; zz < ZC; zz++, x += step) {
         int hi = (int)(x >> 32);
-        bool raw = c.z0 + zz == D - 1;  // last plane: raw voxels
-        if (BLEND && hi >= W - 1) {     // last column: its unblended voxel (column W holds it)
-            hi = W;
-            raw = true;
-        }
-        const bool fp = flip && !raw, in = (unsigned)(zz - z1) < cnt;
+        // raw voxels: the last plane, the last column and beside the volume
+        const bool raw = c.z0 + zz == D - 1 || (unsigned)hi >= (unsigned)(W - 1);
+        if (BLEND && hi >= W - 1) hi = W;  // column W holds the last column's unblended voxel
+        const bool in = (unsigned)(zz - z1) < cnt;
         float g = fix_one_plus_frac((uint32_t)x);
-        g = fp ? 2.0f - g : g - 1.0f;
-        if (raw) g = 0.0f;
+        g = flip ? 2.0f - g : g - 1.0f;
+        if (raw) g = 1.0f;
         const unsigned o = ((unsigned)(zz * pitch) + min((unsigned)(hi - c.cb), most)) << 5;
-        const unsigned oa = o + (fp ? 32u : 0u), ob = o + (fp ? 0u : 32u);
-        add_tap<FL, false>(s, h0 + oa, h0 + ob, h1 + oa, h1 + ob, g, fp, h, in);
+        // a raw voxel v is 0 + 1 (v - 0): exact, and no other column can make it NaN
+        const unsigned oa = raw ? kZeroOff - buf : o + (flip ? 32u : 0u), ob = o + (flip || raw ? 0u : 32u);
+        add_tap<FL, false>(s, h0 + oa, h0 + ob, h1 + oa, h1 + ob, g, flip || raw, h, in);
     }
     settle<FL>(s, flatmask, h);
     return Rows8{{s.p[0], s.p[1], s.p[2], s.p[3]}};
@@ -270,6 +270,7 @@ __device__ __forceinline__ bool fpr_body(const FpLaunch& a, const int g0, const 
             s_base[1] = min(min(hi + 1, H - 1) - lo + 1, a.rv.rawrows);
         }
     }
+    if (tid < 8) *reinterpret_cast<float*>(fsm + kZeroOff + 4 * tid) = 0.0f;
     if (use_tma && tid == 0) {
         mbar_init(bar, 1);
         fence_mbar_init();
