@@ -205,10 +205,10 @@ tomo_status build_plan(tomo_batch* b) {
         const int nsub = (N + upd - 1) / upd;
         b->max_nsub = std::max(b->max_nsub, nsub);
         b->has_fista = b->has_fista || p->fista;
-        // (a member's scratch may grow while its updates are planned: sized first)
+        // the scratch stays where it is once the descriptors point at it: sized first
         for (int T : {upd, N - (nsub - 1) * upd}) {
             FprPlan plan{};
-            handle_fpr_prepare(p, T, &plan);
+            handle_fpr_prepare(p, T, &plan, true);
         }
         b->states.push_back(handle_plan_state(p));
         // rows the forward projector never writes must read as zero residual
@@ -248,7 +248,7 @@ tomo_status build_plan(tomo_batch* b) {
             a.row_off = g.fp_row_off;
             a.status = p->d_status;
             FprPlan plan{};
-            const int tc = handle_fpr_prepare(p, T, &plan);
+            const int tc = handle_fpr_prepare(p, T, &plan, false);
             if (tc > 0) {
                 for (int t0 = 0, c = 0; t0 < T; t0 += tc, c++) {
                     FpLaunch q = a;

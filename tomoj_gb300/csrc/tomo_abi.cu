@@ -25,6 +25,7 @@ namespace {
 thread_local std::string g_err;
 std::atomic<uint64_t> g_in_use{0};
 std::atomic<uint64_t> g_limit{0};
+std::atomic<uint64_t> g_releases{0};  // times device memory was given back or the limit was set
 
 tomo_status fail(tomo_status code, const std::string& msg) {
     g_err = msg;
@@ -152,6 +153,7 @@ void free_n(tomo_projector* p, T** ptr, size_t n) {
     g_in_use -= n * sizeof(T);
     p->bytes -= n * sizeof(T);
     *ptr = nullptr;
+    g_releases++;
 }
 
 // Waits for the handle's stream and reads the status word and, with err, the first T error sums in
@@ -214,6 +216,23 @@ int auto_tilts_per_cta(const tomo_projector* p, int T, int rows) {
     return (T + groups - 1) / groups;
 }
 
+bool capturing(const tomo_projector* p) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(p->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
+}
+
+// Replaces the partial-sum scratch by one of n floats.  The old one is given back only when the
+// new one is there (a refusal leaves it in use), after the work queued on the handle's stream.
+bool grow_fppart(tomo_projector* p, size_t n) {
+    float* fresh = nullptr;
+    if (alloc_n(p, &fresh, n) != TOMO_OK) return false;
+    free_n(p, &p->d_fppart, p->fppart_cap);
+    p->d_fppart = fresh;
+    p->fppart_cap = n;
+    p->plan_gen++;
+    return true;
+}
+
 // Depth split of a forward projection of T tilts over rows [j0, j1): the number of
 // parts, after making sure the scratch exists.  Scratch is only allocated outside
 // stream capture; a captured launch that lacks it runs unsplit.
@@ -227,15 +246,8 @@ int fp_split(tomo_projector* p, int T, int rows, int tpc) {
     const size_t need_part = (size_t)P * T * p->npix;
     const size_t need_tk = (size_t)groups * g.h;
     if (need_part <= p->fppart_cap && need_tk <= p->tickets_cap) return P;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(p->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return 1;
-    if (need_part > p->fppart_cap) {
-        free_n(p, &p->d_fppart, p->fppart_cap);
-        p->fppart_cap = 0;
-        p->plan_gen++;
-        if (alloc_n(p, &p->d_fppart, need_part) != TOMO_OK) return 1;
-        p->fppart_cap = need_part;
-    }
+    if (capturing(p)) return 1;
+    if (need_part > p->fppart_cap && !grow_fppart(p, need_part)) return 1;
     if (need_tk > p->tickets_cap) {
         free_n(p, &p->d_tickets, p->tickets_cap);
         p->tickets_cap = 0;
@@ -250,10 +262,13 @@ int fp_split(tomo_projector* p, int T, int rows, int tpc) {
 // The segment sums of a launch take at most eight times the series' size (the handle holds
 // six such buffers) and 1 GiB, or half the bytes of an FP32 volume where that is more (every launch
 // reads the volume again: a SIRT iteration of 2048 x 512 x 2048 with 121 tilts takes 176 ms in launches
-// of five tilts, 161 ms in launches of 24); more tilts run in further launches.  Memory that is
-// refused leaves the 1 GiB, then the one-row form.  Volumes that hold NaN or Inf stay on the
-// one-row form, whose samples treat them as before.
-int fpr_prepare(tomo_projector* p, int T, FprPlan* plan) {
+// of five tilts, 161 ms in launches of 24); more tilts run in further launches, which changes no
+// sum.  Where memory is refused, scratch of half as many tilts is tried and so on, down to what the
+// handle holds; the one-row form is left for a handle that cannot hold one tilt's sums.  A refused
+// size is not tried again before some device memory has been given back (g_releases).  Volumes that
+// hold NaN or Inf stay on the one-row form, whose samples treat them as before.
+// grow: the scratch may be replaced (never under capture, nor where other streams may use it).
+int fpr_prepare(tomo_projector* p, int T, FprPlan* plan, bool grow = true) {
     const Geometry& g = p->g;
     if (T <= 0 || !g.separable || p->vol_flag()) return 0;
     FprGeom fg{g.W, g.H, g.D, g.w, g.h, p->vtype, p->fp_max_step, p->fp_max_space, p->fp_min_space,
@@ -269,31 +284,25 @@ int fpr_prepare(tomo_projector* p, int T, FprPlan* plan) {
     *plan = *have;
     if (plan->zc == 0) return 0;
     const size_t per_tilt = (size_t)plan->nseg * p->npix;
-    const size_t base = (size_t)1 << 28;
-    auto tilts = [&](size_t room) {
-        const size_t lim = std::min<size_t>((size_t)8 * g.N * p->npix, room);
-        int tc = (int)std::min<size_t>((size_t)T, std::max<size_t>(1, lim / per_tilt));
-        if (tc < T && tc >= plan->tg) tc -= tc % plan->tg;
-        return tc;
-    };
-    int tc = tilts(p->fpr_denied ? base : std::max(base, p->nvox / 2));
-    if (p->tilts_per_cta > 0) plan->tg = std::min({p->tilts_per_cta, kFprMaxTilts, T});
-    const size_t need = per_tilt * (size_t)tc;
-    if (need > p->fppart_cap) {
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(p->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return 0;
-        free_n(p, &p->d_fppart, p->fppart_cap);
-        p->fppart_cap = 0;
-        p->plan_gen++;
-        size_t got = need;
-        if (alloc_n(p, &p->d_fppart, got) != TOMO_OK) {
-            p->fpr_denied = true;
-            tc = tilts(base);
-            got = per_tilt * (size_t)tc;
-            if (got >= need || alloc_n(p, &p->d_fppart, got) != TOMO_OK) return 0;
+    const size_t room = std::max((size_t)1 << 28, p->nvox / 2);
+    const size_t lim = std::min<size_t>((size_t)8 * g.N * p->npix, room);
+    // whole CTAs of tilts
+    auto whole = [&](int tc) { return tc < T && tc >= plan->tg ? tc - tc % plan->tg : tc; };
+    const int want = whole((int)std::min<size_t>((size_t)T, std::max<size_t>(1, lim / per_tilt)));
+    int tc = want;
+    if (grow && per_tilt * (size_t)tc > p->fppart_cap && !capturing(p)) {
+        if (p->fpr_refused_at != g_releases.load()) p->fpr_refused = SIZE_MAX;
+        size_t refused = p->fpr_refused;
+        for (int t = tc; t >= 1 && per_tilt * (size_t)t > p->fppart_cap; t = whole(t / 2)) {
+            if (per_tilt * (size_t)t >= refused) continue;
+            if (grow_fppart(p, per_tilt * (size_t)t)) break;
+            refused = per_tilt * (size_t)t;
         }
-        p->fppart_cap = got;
+        p->fpr_refused = refused;
+        p->fpr_refused_at = g_releases.load();
     }
+    tc = whole((int)std::min<size_t>((size_t)want, p->fppart_cap / per_tilt));
+    if (p->tilts_per_cta > 0) plan->tg = std::min({p->tilts_per_cta, kFprMaxTilts, T});
     return tc;
 }
 
@@ -316,7 +325,7 @@ tomo_status ensure_fp_rowmap(tomo_projector* p, int j0) {
 // row-stream iteration).
 tomo_status launch_fp(tomo_projector* p, FpLaunch a, bool whole = false) {
     FprPlan plan{};
-    const int tc = fpr_prepare(p, a.T, &plan);
+    const int tc = fpr_prepare(p, a.T, &plan, !whole);
     if (tc > 0) {
         const int T = a.T;
         a.rv = plan;
@@ -677,7 +686,7 @@ tomo_status handle_need_series(tomo_projector* p) { return need_series(p); }
 tomo_status handle_start_iteration(tomo_projector* p) { return start_iteration(p); }
 tomo_status handle_end_iteration(tomo_projector* p) { return end_iteration(p); }
 int handle_tilts_per_cta(const tomo_projector* p, int T) { return auto_tilts_per_cta(p, T, 0); }
-int handle_fpr_prepare(tomo_projector* p, int T, FprPlan* plan) { return fpr_prepare(p, T, plan); }
+int handle_fpr_prepare(tomo_projector* p, int T, FprPlan* plan, bool grow) { return fpr_prepare(p, T, plan, grow); }
 }  // namespace tomo
 
 extern "C" {
@@ -687,6 +696,7 @@ const char* tomo_last_error(void) { return g_err.c_str(); }
 
 tomo_status tomo_set_memory_limit(uint64_t bytes) {
     g_limit = bytes;
+    g_releases++;
     return TOMO_OK;
 }
 uint64_t tomo_memory_in_use(void) { return g_in_use.load(); }
@@ -842,6 +852,7 @@ tomo_status tomo_destroy(tomo_projector* p) {
         for (void* a : p->allocs) dfree(a, d ? d->stream : nullptr);
     }
     g_in_use -= p->bytes;
+    g_releases++;
     for (cudaEvent_t e : p->rs_ev) cudaEventDestroy(e);
     for (cudaStream_t q : p->rs)
         if (q) cudaStreamDestroy(q);

@@ -1,6 +1,7 @@
 // The projector handle (shared by the C-ABI translation units).
 #pragma once
 #include <atomic>
+#include <cstdint>
 #include <utility>
 #include <vector>
 
@@ -139,7 +140,8 @@ struct tomo_projector {
     // forward-projector depth split scratch (partial ray sums, per-group tickets)
     float* d_fppart = nullptr;
     size_t fppart_cap = 0;  // floats
-    bool fpr_denied = false;  // the larger scratch of the row-vector projector was refused
+    size_t fpr_refused = SIZE_MAX;  // smallest scratch of the row-vector projector that was refused (floats)
+    uint64_t fpr_refused_at = 0;    // g_releases then
     unsigned* d_tickets = nullptr;
     size_t tickets_cap = 0;
     // per-kernel timing of the OS-SART driver (tomo_set_profiling)
@@ -166,6 +168,7 @@ inline std::pair<uint64_t, bool> handle_plan_state(tomo_projector* p) { return {
 int handle_tilts_per_cta(const tomo_projector* p, int T);
 // Plan of the row-vector forward projector for updates of T tilts and the tilts one launch
 // takes (the partial sums' scratch is bounded); 0: the handle's projections run the one-row
-// form.  Allocates the scratch unless the handle's stream is being captured.
-int handle_fpr_prepare(tomo_projector* p, int T, tomo::FprPlan* plan);
+// form.  With grow, makes the scratch larger where it can, unless the handle's stream is being
+// captured.
+int handle_fpr_prepare(tomo_projector* p, int T, tomo::FprPlan* plan, bool grow);
 }  // namespace tomo
