@@ -168,15 +168,38 @@ __device__ __forceinline__ void add2(F2& s, float p, float pe) {
     s.hi = t;
 }
 
+// Whether a pair of floats holds the square of a difference q * factor of magnitude m (not where m
+// is NaN: an extreme factor, see fpr_split_factor).
+__device__ __forceinline__ bool pair_range(float m, float q) { return m <= 1e15f && (m >= 1e-15f || q == 0.0f); }
+
+// The differences of projection row j of batch slot b that pair_range leaves out, in double: written
+// again, squares returned.  Over this thread's columns; out of line and from the projections and norms
+// it has written, so that the pass itself carries nothing for them.
+__device__ __noinline__ double far_row(const FpLaunch& a, int b, int tilt, int j) {
+    double sum = 0.0;
+    for (int i = threadIdx.x; i < a.w; i += kFinishThreads) {
+        const size_t o = ((size_t)b * a.h + j) * a.w + i;
+        const float e = a.meas[((size_t)tilt * a.h + j) * a.w + i], th = a.proj[o];
+        if (isnan(e) || isnan(th)) continue;
+        const float q = __fdiv_rn(__fsub_rn(e, th), a.norm[o]);
+        if (pair_range(fabsf(mul_split(q, F2{a.factor_hi, a.factor_lo}).hi), q)) continue;
+        const double x = (double)q * a.factor;
+        a.diff[o] = __double2float_rn(x);
+        sum += x * x;
+    }
+    return sum;
+}
+
 // Projection, norm, difference and residual of n <= RJ consecutive projection rows from their
 // segment sums (the epilogue of fp_body with the sums read back, in segment order).  The
-// squared differences are summed in FP32 pairs with error terms, a warp's sums in FP64; a
-// row's order of adds depends on neither RJ nor UC.  Bound by its memory traffic (segment
+// squared differences are summed in FP32 pairs with error terms (those outside a pair's range
+// in FP64 by far_row), a warp's sums in FP64; a row's order of adds depends on neither RJ nor UC.  Bound by its memory traffic (segment
 // sums, measured row in; projection, norm and difference out) when RJ rows share a ray's
 // 32-byte table entry, and by latency on grids of few rows, where UC columns of a row are
 // read at once instead.  One row and one column at a time took 13 us for 7 tilts of 512 x 256
 // in 5 segments, 482 us for 61 of 1024 x 1024 and 339 us for 12 series of 61 x 512 x 64;
-// these forms take 12, 374 and 284 us (two rows: 394 and 299 us for the last two).
+// these forms take 12, 352 and 278 us (two rows: 394 and 299 us for the last two; with the
+// differences outside the pairs' range in the same loop 377 and 283 us).
 template <int RJ, int UC>
 __device__ __forceinline__ void finish_rows(const FpLaunch& a, int b, int j0, int n) {
     __shared__ double red[RJ][kFinishThreads / 32];
@@ -187,7 +210,7 @@ __device__ __forceinline__ void finish_rows(const FpLaunch& a, int b, int j0, in
     bool row_in[RJ];
     float vsc[RJ];
     F2 e2[RJ];
-    double far[RJ];  // squares outside FP32's comfortable range
+    bool any_far = false;  // a difference of this thread lies outside the pairs' range
 #pragma unroll
     for (int y = 0; y < RJ; y++) {
         const int r = y >= n ? -1 : a.two_rows ? a.rowmap[j0 + y] : j0 + y - a.row_off;
@@ -195,7 +218,6 @@ __device__ __forceinline__ void finish_rows(const FpLaunch& a, int b, int j0, in
         // reduced storage: ray sums are in units of the row's slab scale (a power of two)
         vsc[y] = (a.vscale != nullptr && row_in[y]) ? a.vscale[r] : 1.0f;
         e2[y] = F2{0.0f, 0.0f};
-        far[y] = 0.0;
     }
     for (int i0 = threadIdx.x; i0 < a.w; i0 += kFinishThreads * UC) {
         float e[UC][RJ], sum[UC][RJ], nrm[UC];
@@ -253,7 +275,7 @@ __device__ __forceinline__ void finish_rows(const FpLaunch& a, int b, int j0, in
                 const size_t o = row + (size_t)y * a.w + i;
                 float th = __int_as_float(0x7fc00000), nr = 0.0f;
                 if (s1[c] >= 0 && row_in[y]) {
-                    th = mul_split(sum[c][y] * vsc[y], ninc).hi;
+                    th = mul_split(sum[c][y], ninc).hi * vsc[y];
                     nr = nrm[c];
                 }
                 a.proj[o] = th;
@@ -261,14 +283,15 @@ __device__ __forceinline__ void finish_rows(const FpLaunch& a, int b, int j0, in
                 if (a.meas != nullptr) {
                     float d = 0.0f;
                     if (!isnan(e[c][y]) && !isnan(th)) {
-                        const F2 v = mul_split(__fdiv_rn(__fsub_rn(e[c][y], th), nr), fac);
+                        const float q = __fdiv_rn(__fsub_rn(e[c][y], th), nr);
+                        const F2 v = mul_split(q, fac);
                         d = v.hi;
                         const float m = fabsf(d);
-                        if ((m > 1e15f || m < 1e-15f) && d != 0.0f) {
-                            far[y] += (double)d * d;
-                        } else {
+                        if (pair_range(m, q)) {
                             const float p = d * d;
                             add2(e2[y], p, fmaf(d, d, -p) + 2.0f * d * v.lo);
+                        } else {
+                            any_far = true;
                         }
                     }
                     a.diff[o] = d;
@@ -279,17 +302,17 @@ __device__ __forceinline__ void finish_rows(const FpLaunch& a, int b, int j0, in
     if (a.meas != nullptr) {
 #pragma unroll
         for (int y = 0; y < RJ; y++) {
-            // the lanes' sums in fixed order, without FP64 (an infinite sum has no error term)
+            // the lanes' sums in fixed order, without FP64
 #pragma unroll
             for (int q = 16; q > 0; q >>= 1) {
                 const float oh = __shfl_down_sync(0xffffffffu, e2[y].hi, q);
                 const float ol = __shfl_down_sync(0xffffffffu, e2[y].lo, q);
                 add2(e2[y], oh, ol);
             }
-            if (__any_sync(0xffffffffu, far[y] != 0.0)) far[y] = warp_sum(far[y]);
+            double far = 0.0;
+            if (__any_sync(0xffffffffu, any_far)) far = warp_sum(any_far && y < n ? far_row(a, b, tilt, j0 + y) : 0.0);
             if ((threadIdx.x & 31) == 0)
-                red[y][threadIdx.x >> 5] =
-                    (isfinite(e2[y].hi) ? (double)e2[y].hi + (double)e2[y].lo : (double)e2[y].hi) + far[y];
+                red[y][threadIdx.x >> 5] = (double)e2[y].hi + (double)e2[y].lo + far;
         }
         __syncthreads();
         if (threadIdx.x < n) {
@@ -436,8 +459,10 @@ int fpr_row_groups(const FpLaunch& a, int* jfirst) {
 }
 
 void fpr_split_factor(FpLaunch* a) {
-    a->factor_hi = (float)a->factor;
-    a->factor_lo = std::isfinite(a->factor_hi) ? (float)(a->factor - (double)a->factor_hi) : 0.0f;
+    const double m = std::fabs(a->factor);
+    const bool fits = m == 0.0 || (m >= 0x1p-60 && m <= 0x1p60);  // both parts, and products with them, normal
+    a->factor_hi = fits ? (float)a->factor : NAN;
+    a->factor_lo = fits ? (float)(a->factor - (double)a->factor_hi) : 0.0f;
 }
 
 cudaError_t launch_fpr(const FpLaunch& a0, cudaStream_t s) {

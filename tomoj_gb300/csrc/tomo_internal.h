@@ -153,7 +153,7 @@ struct FpLaunch {
     float* diff;            // [T][h][w] (written when meas != nullptr)
     double* errpart;        // [T][h] per-row sum of squared differences
     double factor;          // relaxation factor passed to projectAndDifference
-    float factor_hi, factor_lo;  // factor as a sum of two floats (row-vector form)
+    float factor_hi, factor_lo;  // factor as a sum of two floats (row-vector form; NaN: only the double will do)
     int j0, j1;             // projection rows to compute
     int tilts_per_cta;
     int W, H, D, w, h;
