@@ -59,14 +59,18 @@ __device__ __forceinline__ FPair pair_lerp(FPair a, FPair b, FPair t) {
     return r;
 }
 
-// One pixel from 64-bit fixed-point coordinates (2^-48 pixel) and bilinear weights and sums in
-// pairs of floats, rounded once at the end: what double arithmetic gives to a few parts in
-// 2^46.  0: outside, 1: *pix set, 2: not decided here (a coordinate within 2^-20 of a whole
+// One pixel from 64-bit fixed-point coordinates (known to 2^-47 pixel: steps of 2^-64, so that
+// thousands of columns and rows add nothing; the double expressions round to 2^-40 at x = 4096) and
+// bilinear weights and sums in pairs of floats (a few parts in 2^46 of the largest neighbour),
+// rounded once at the end.  F: whole parts in units of 2^-48, then the rest in units of 2^-64.
+// 0: outside, 1: *pix set, 2: not decided here (a coordinate within 2^-20 of a whole
 // pixel, where truncation is the reference's double rounding's, or neighbours that are not
 // finite, or so large or small that a pair would lose bits).
 __device__ __forceinline__ int align_pixel_fixed(const float* __restrict__ un, const long long* __restrict__ F, int md,
                                                  int i, int j, int w, int h, float* pix) {
-    const long long X = F[0] * i + F[2] * j + F[4], Y = F[1] * i + F[3] * j + F[5];
+    // (rests below 2^16, columns + rows at most 2^16: the sum fits 32 bits)
+    auto rest = [&](int k) { return ((unsigned)F[6 + k] * i + (unsigned)F[8 + k] * j + (unsigned)F[10 + k]) >> 16; };
+    const long long X = F[0] * i + F[2] * j + F[4] + rest(0), Y = F[1] * i + F[3] * j + F[5] + rest(1);
     constexpr long long kOne = 1LL << 48, kNear = 1LL << 28;
     const long long nx = md & 4 ? 0 : kNear, ny = md & 8 ? 0 : kNear;
     if (((X + nx) & (kOne - 1)) < 2 * nx || ((Y + ny) & (kOne - 1)) < 2 * ny) return 2;
@@ -95,11 +99,11 @@ __device__ __forceinline__ int align_pixel_fixed(const float* __restrict__ un, c
 }
 
 // mode per image: 0 double expressions, 1 identity, 2 fixed-point coordinates (fix: {x, y per
-// column, x, y per row, x, y at pixel (0, 0)} times 2^48) with + 4 and + 8 where x and y are
+// column, x, y per row, x, y at pixel (0, 0)} in two parts, see align_pixel_fixed) with + 4 and + 8 where x and y are
 // exact in both forms (whole or dyadic shifts).  flags: bit 0 a NaN was written, bit 1 an
 // infinity, bit 2 set where a pixel took the fill.  This part's FP64 rate is 1/64 of FP32: 61 images of 512 x 256 took 628
-// us in doubles and take 65 us in fixed point and float pairs, with the scan for
-// non-finite pixels (9 us) in the same pass.
+// us in doubles and take 69 us in fixed point and float pairs, with the scan for
+// non-finite pixels (9 us) in the same pass (66 us without the steps' second parts).
 constexpr int kAlignPix = 4;  // pixels per thread
 
 __global__ void __launch_bounds__(256) align_kernel(const float* __restrict__ raw, float* __restrict__ out,
@@ -127,7 +131,7 @@ __global__ void __launch_bounds__(256) align_kernel(const float* __restrict__ ra
         } else {
             const int j = e >> 32 ? (int)(e / w) : (int)((unsigned)e / (unsigned)w), i = (int)(e - (size_t)j * w);
             int st = 2;
-            if (md & 2) st = align_pixel_fixed(un, fix + 6 * t, md, i, j, w, h, &pix);
+            if (md & 2) st = align_pixel_fixed(un, fix + 12 * t, md, i, j, w, h, &pix);
             if (st == 2) in = align_pixel_exact(un, tinv + 6 * t, i, j, w, h, &pix);
             else in = st == 1;
         }

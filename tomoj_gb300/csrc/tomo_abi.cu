@@ -778,7 +778,7 @@ tomo_status tomo_create(const tomo_geom* geom, const tomo_params* params, tomo_p
     A(alloc_n(p, &p->d_btilt, N));
     A(alloc_n(p, &p->d_zint, N * g.W));
     A(alloc_n(p, &p->d_tinv, N * 6));
-    A(alloc_n(p, &p->d_tfix, N * 6));
+    A(alloc_n(p, &p->d_tfix, N * 12));
     A(alloc_n(p, &p->d_stats, N * 2));
     A(alloc_n(p, &p->d_identity, N));
     A(alloc_n(p, &p->d_mask, (size_t)g.w));
@@ -994,7 +994,7 @@ tomo_status tomo_load_series(tomo_projector* p, const float* pixels, int32_t pix
     CKS(setup_geometry(p));
     // alignment: Tinv = AffineTransform.createInverse (general case)
     std::vector<double> tinv((size_t)N * 6), st((size_t)N * 2);
-    std::vector<long long> tfix((size_t)N * 6);
+    std::vector<long long> tfix((size_t)N * 12);
     std::vector<unsigned char> ident(N);
     for (int t = 0; t < N; t++) {
         double T[6] = {1, 0, 0, 1, 0, 0};
@@ -1012,19 +1012,31 @@ tomo_status tomo_load_series(tomo_projector* p, const float* pixels, int32_t pix
         I[4] = (m01 * m12 - m11 * m02) / det;
         I[5] = (m10 * m02 - m00 * m12) / det;
         // fixed-point coordinates of pixel (i, j): (I00, I01) and (I10, I11) per column and row,
-        // the rest at (0, 0); used where every coordinate of the image stays below 2^14
+        // the rest at (0, 0); used where every coordinate of the image stays below 2^14 (and its
+        // columns and rows below 2^16)
         const double cx = g.w / 2.0, cy = g.h / 2.0;
         const double o[2] = {I[4] + cx - I[0] * cx - I[2] * cy, I[5] + cy - I[1] * cx - I[3] * cy};
-        long long* F = &tfix[6 * (size_t)t];
-        bool fits = true;
+        long long* F = &tfix[12 * (size_t)t];
+        bool fits = g.w + g.h <= 65536;
         for (int k = 0; k < 2; k++) {
             const double reach = std::fabs(I[k]) * g.w + std::fabs(I[2 + k]) * g.h + std::fabs(o[k]);
             fits = fits && reach < 16384.0;  // false for NaN
         }
-        for (int k = 0; k < 2 && fits; k++) {
-            F[k] = std::llrint(I[k] * 281474976710656.0);
-            F[2 + k] = std::llrint(I[2 + k] * 281474976710656.0);
-            F[4 + k] = std::llrint(o[k] * 281474976710656.0);
+        if (fits) {
+            // in units of 2^-64 (products with powers of two and the remainder are exact)
+            auto fixed = [](double v) -> __int128 {
+                const double whole = std::rint(v * 0x1p48);
+                return ((__int128)(long long)whole << 16) + (__int128)std::llrint((v * 0x1p48 - whole) * 65536.0);
+            };
+            for (int k = 0; k < 2; k++) {
+                const __int128 col = fixed(I[k]), row = fixed(I[2 + k]);
+                const __int128 at0 = fixed(I[4 + k]) + ((((__int128)(k ? g.h : g.w) << 64) - col * g.w - row * g.h) >> 1);
+                const __int128 c[3] = {col, row, at0};
+                for (int q = 0; q < 3; q++) {
+                    F[2 * q + k] = (long long)(c[q] >> 16);
+                    F[6 + 2 * q + k] = (long long)(c[q] & 0xFFFF);
+                }
+            }
         }
         int mode = fits ? 2 : 0;
         for (int k = 0; k < 2 && fits; k++) {

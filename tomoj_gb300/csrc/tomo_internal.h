@@ -288,7 +288,7 @@ int bp_segment_pairs(bool wide);
 // Aligned images (fix, mode: see align_kernel; |coordinates| below 2^14 for mode & 2); *flags
 // (zeroed by the caller) receives bit 0 for a NaN, bit 1 for an infinity among them, bit 2 where a
 // pixel took the fill.
-cudaError_t launch_align(const float* raw, float* out, const double* tinv /*[N][6]*/, const long long* fix /*[N][6]*/,
+cudaError_t launch_align(const float* raw, float* out, const double* tinv /*[N][6]*/, const long long* fix /*[N][12]*/,
                          const double* stats, int N, int w, int h, int normalize, int fill, const unsigned char* mode,
                          int* flags, cudaStream_t s);
 // Row filters: mask_row and H lie in the order in which the in-place passes leave the
