@@ -284,6 +284,14 @@ tomo_status tomo_batch_iteration(tomo_batch* b, const double* relax, const int32
  * accumulated since profiling was enabled. */
 tomo_status tomo_set_profiling(tomo_projector* p, int32_t enabled);
 tomo_status tomo_profile_read(tomo_projector* p, double* out4);
+/* How the forward projection of an update of `update` tilts (0: all) of such a series is cut
+ * (no counterpart in the reference; needs no handle, and no GPU: 152 multiprocessors are
+ * taken then): out8 = {planes per chunk, planes per segment, segments, column windows,
+ * columns of a plane buffer, tilts per CTA, tilts per launch, bytes of the scratch a handle
+ * takes for it at its first projection while memory is not short}; zeros where the series
+ * does not run on the row-vector form. */
+tomo_status tomo_projection_plan(const tomo_geom* geom, int32_t precision, const double* euler, int32_t update,
+                                 int64_t* out8);
 /* Tilts per forward-projection CTA (0 = automatic; tuning knob). */
 tomo_status tomo_set_tilts_per_cta(tomo_projector* p, int32_t n);
 /* Volume rows per backprojection thread (tuning knob, no counterpart in the reference):

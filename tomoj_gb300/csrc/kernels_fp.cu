@@ -4,8 +4,6 @@
 // (QP = ceil(w / threads); kernel in fp_kernel.cuh, one per (threads, QP) in fp_kernel_q*.cu).
 #include <algorithm>
 #include <cmath>
-#include <functional>
-#include <queue>
 #include <vector>
 
 #include "device_util.cuh"
@@ -340,32 +338,60 @@ __global__ void __launch_bounds__(kFinishThreads, 8)
 
 size_t fpr_smem_bytes(const FprPlan& p) { return kFprFixedSmem + (size_t)p.zc * p.pitch * (64 + 4 * p.rawrows); }
 
-// Time of a grid on `sms` SMs in units of a full segment's CTA: CTAs start in segment order,
-// `per_seg` each.  A segment away from the middle plane has fewer rays inside, the last one
-// fewer planes.
-static double grid_time(int nseg, int per_seg, double last, double lean, int sms) {
-    const double n = (double)nseg * per_seg;
-    auto weight = [&](int s) {
+// A grid on `sms` SMs: CTAs start in segment order, `per_seg` each.  Times are in units of a full
+// segment's CTA; a segment away from the middle plane has fewer rays inside, the last one fewer
+// planes.
+namespace {
+struct CtaGrid {
+    int nseg, per_seg, sms;
+    double last, lean;
+    double weight(int s) const {
         const double d = nseg > 1 ? std::fabs((s + 0.5) / nseg - 0.5) * 2 : 0.0;
         return (s == nseg - 1 ? last : 1.0) * (1.0 - lean * d);
-    };
-    if (n > 4.0 * sms) {
-        double sum = 0;
-        for (int s = 0; s < nseg; s++) sum += weight(s);
-        return sum * per_seg / sms + 0.5;
     }
-    std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
-    for (int k = 0; k < sms; k++) free_at.push(0.0);
-    double end = 0;
-    for (int s = 0; s < nseg; s++)
-        for (int k = 0; k < per_seg; k++) {
-            const double t = free_at.top() + weight(s);
-            free_at.pop();
-            free_at.push(t);
-            end = std::max(end, t);
+    bool many() const { return (double)nseg * per_seg > 4.0 * sms; }
+    // work per SM: the time of many CTAs, less half a CTA.  (The distances of weight() add up to
+    // nseg / 2, less 1 / (2 nseg) for odd numbers of segments.)
+    double mean() const {
+        const double dist = nseg > 1 ? 0.5 * nseg - (nseg & 1 ? 0.5 / nseg : 0.0) : 0.0;
+        const double first = nseg > 1 ? weight(0) : 1.0;  // the last one's, were it full
+        return (nseg - lean * dist - first + weight(nseg - 1)) * per_seg / sms;
+    }
+    // No grid of few CTAs is faster: the mean, and the busiest SM's CTAs at the shortest times there are.
+    double least() const {
+        const double end = weight(nseg - 1), other = nseg > 1 ? weight(0) : end;
+        const int rounds = (int)(((long long)nseg * per_seg + sms - 1) / sms);
+        const int ends = end < other ? std::min(per_seg, rounds) : 0;
+        return std::max(mean(), ends * end + (rounds - ends) * std::min(other, end >= other ? end : other)) * (1.0 - 1e-9);
+    }
+    // Few CTAs, each taken by the SM that is free first.
+    double simulated() const {
+        std::vector<double> free_at(sms, 0.0);  // a binary heap, earliest first
+        const long long n = (long long)nseg * per_seg;
+        long long k = 0;
+        double end = 0;
+        for (int s = 0; s < nseg; s++) {
+            const double w = weight(s);
+            for (int q = 0; q < per_seg; q++, k++) {
+                if (n <= sms) {  // an SM for every CTA
+                    end = std::max(end, w);
+                    break;
+                }
+                const double t = free_at[0] + w;
+                end = std::max(end, t);
+                int i = 0;
+                for (int c; (c = 2 * i + 1) < sms; i = c) {
+                    if (c + 1 < sms && free_at[c + 1] < free_at[c]) c++;
+                    if (free_at[c] >= t) break;
+                    free_at[i] = free_at[c];
+                }
+                free_at[i] = t;
+            }
         }
-    return end;
-}
+        return end;
+    }
+};
+}  // namespace
 
 // Cuts a projection into CTAs by a cost model (cycles of one SM): a plane costs half a cycle
 // per staged column (8 voxels transposed at 16 a cycle) and 18.4 cycles per ray block (256
@@ -376,6 +402,10 @@ static double grid_time(int nseg, int per_seg, double last, double lean, int sms
 // 1024 x 256 x 256, 61 tilts in 6 windows of 3 segments 1567 us, 5 of 3 1655 us.
 // Deeper chunks leave narrower windows (the buffers hold zc * pitch columns), longer segments
 // wider margins around a window (tilts fan out by max_step columns per plane).
+// The first projection of a handle waits for this (a 128 x 32 x 128 update takes 98 us), so grids
+// of few CTAs, whose time takes a simulation, are looked at in the order of their lower bounds and
+// only while one could still be the cheapest: the choice is that of simulating all, in 1 to 25 us
+// instead of 30 to 118 (256 x 64 x 256, 61 tilts).
 FprPlan fpr_plan(const FprGeom& g, int T, int sms) {
     FprPlan best{};
     if (T <= 0 || g.w > 4096 || !(g.max_step <= 16.0) || !(g.max_space <= 64.0) || !(g.min_space > 0)) return best;
@@ -384,7 +414,13 @@ FprPlan fpr_plan(const FprGeom& g, int T, int sms) {
     const int rawrows = g.row_step > 0 ? (int)std::ceil(7 * g.row_step) + 2 : 8;
     if (rawrows > 16) return best;
     const int nrg = (g.rows + 14) / 8;
-    double best_cost = 0;
+    struct Cut {
+        FprPlan p;
+        CtaGrid grid;
+        double unit, rest, cost;  // cycles per unit of grid time and besides; cost or its lower bound
+    };
+    std::vector<Cut> cuts;
+    cuts.reserve(72);
     for (int zc : {8, 6, 4}) {
         const int room = (int)((kFprSmemMax - kFprFixedSmem) / ((size_t)zc * (64 + 4 * rawrows)));
         for (int nch = 1; nch <= kFprMaxChunks; nch = nch < 8 ? nch + 1 : nch + (nch + 3) / 4) {
@@ -431,17 +467,29 @@ FprPlan fpr_plan(const FprGeom& g, int T, int sms) {
             per_plane = std::max(per_plane, 1200.0 / zc) + 600.0 / zc;
             const double last = (double)(g.D - (p.nseg - 1) * seg) / seg;
             const double lean = std::min(0.35, 0.2 * g.D * g.max_step / g.W);
-            const double cost = grid_time(p.nseg, ntg * p.nwin * nrg, last, lean, sms) *
-                                    (std::min(seg, g.D) * per_plane + 12000.0) +
-                                (double)p.nseg * T * g.h * g.w * 8.0 / 3400.0;
-            if (best.zc == 0 || cost < best_cost) {
-                best = p;
-                best_cost = cost;
-            }
+            Cut c{p, CtaGrid{p.nseg, ntg * p.nwin * nrg, sms, last, lean}, std::min(seg, g.D) * per_plane + 12000.0,
+                  (double)p.nseg * T * g.h * g.w * 8.0 / 3400.0, 0.0};
+            c.cost = (c.grid.many() ? c.grid.mean() + 0.5 : c.grid.least()) * c.unit + c.rest;
+            cuts.push_back(c);
             if (seg >= g.D) break;
         }
     }
-    return best;
+    if (cuts.empty()) return best;
+    // cheapest first (of equal ones the first listed): done when the cheapest cost is exact
+    auto dearer = [&](int x, int y) { return cuts[x].cost != cuts[y].cost ? cuts[x].cost > cuts[y].cost : x > y; };
+    std::vector<int> order(cuts.size());
+    for (size_t i = 0; i < order.size(); i++) order[i] = (int)i;
+    std::make_heap(order.begin(), order.end(), dearer);
+    std::vector<bool> exact(cuts.size(), false);
+    for (;;) {
+        const int i = order.front();
+        Cut& c = cuts[i];
+        if (exact[i] || c.grid.many()) return c.p;
+        std::pop_heap(order.begin(), order.end(), dearer);
+        c.cost = c.grid.simulated() * c.unit + c.rest;
+        exact[i] = true;
+        std::push_heap(order.begin(), order.end(), dearer);
+    }
 }
 
 int fpr_row_groups(const FpLaunch& a, int* jfirst) {

@@ -258,6 +258,44 @@ int fp_split(tomo_projector* p, int T, int rows, int tpc) {
     return P;
 }
 
+// What the tilts of a series make of its geometry: g.separable and g.fractional (vertical-axis tilts
+// run on the XZ-plane kernels; rows that are not a whole row apart, scale != 1 or half-row centre
+// offsets, blend two rows, 16-bit volumes excepted), and the extremes of its rays.
+void classify_tilts(Geometry& g, const double* euler, int vtype, double* max_step, double* max_space, double* min_space) {
+    bool integral = true, vertical = true;
+    for (int t = 0; t < g.N; t++) {
+        integral = integral && tilt_is_separable(euler + 9 * t, g);
+        vertical = vertical && tilt_is_vertical(euler + 9 * t);
+    }
+    g.separable = integral || (vertical && vtype == kVolF32);
+    g.fractional = g.separable && !integral;
+    *max_step = *max_space = 0;
+    *min_space = 1e30;
+    for (int t = 0; t < g.N && g.separable; t++) {
+        const double* R = euler + 9 * t;
+        const double space = 1.0 / std::fabs(R[0] * g.scale);
+        *max_step = std::max(*max_step, std::fabs(R[2] / R[0]));
+        *max_space = std::max(*max_space, space);
+        *min_space = std::min(*min_space, space);
+    }
+}
+
+FprGeom fpr_geom(const Geometry& g, int vtype, double max_step, double max_space, double min_space) {
+    return FprGeom{g.W, g.H, g.D, g.w, g.h, vtype, max_step, max_space, min_space, g.fractional ? g.h : g.H,
+                   g.fractional ? 1.0 / g.scale : 0.0};
+}
+
+// Whole CTAs of tilts.
+int fpr_whole(const FprPlan& plan, int T, int tc) { return tc < T && tc >= plan.tg ? tc - tc % plan.tg : tc; }
+
+// Tilts of T one launch takes while memory is not short.
+int fpr_tilts_per_launch(const Geometry& g, const FprPlan& plan, int T) {
+    const size_t npix = (size_t)g.w * g.h, nvox = (size_t)g.W * g.H * g.D;
+    const size_t lim = std::min<size_t>((size_t)8 * g.N * npix, std::max((size_t)1 << 28, nvox / 2));
+    const size_t per_tilt = (size_t)plan.nseg * npix;
+    return fpr_whole(plan, T, (int)std::min<size_t>((size_t)T, std::max<size_t>(1, lim / per_tilt)));
+}
+
 // Row-vector form: its plan for T tilts and the tilts per launch (see handle_fpr_prepare).
 // The segment sums of a launch take at most eight times the series' size (the handle holds
 // six such buffers) and 1 GiB, or half the bytes of an FP32 volume where that is more (every launch
@@ -271,8 +309,7 @@ int fp_split(tomo_projector* p, int T, int rows, int tpc) {
 int fpr_prepare(tomo_projector* p, int T, FprPlan* plan, bool grow = true) {
     const Geometry& g = p->g;
     if (T <= 0 || !g.separable || p->vol_flag()) return 0;
-    FprGeom fg{g.W, g.H, g.D, g.w, g.h, p->vtype, p->fp_max_step, p->fp_max_space, p->fp_min_space,
-               g.fractional ? g.h : g.H, g.fractional ? 1.0 / g.scale : 0.0};
+    const FprGeom fg = fpr_geom(g, p->vtype, p->fp_max_step, p->fp_max_space, p->fp_min_space);
     const FprPlan* have = nullptr;
     for (auto& q : p->fpr_plans)
         if (q.first == T) have = &q.second;
@@ -284,16 +321,12 @@ int fpr_prepare(tomo_projector* p, int T, FprPlan* plan, bool grow = true) {
     *plan = *have;
     if (plan->zc == 0) return 0;
     const size_t per_tilt = (size_t)plan->nseg * p->npix;
-    const size_t room = std::max((size_t)1 << 28, p->nvox / 2);
-    const size_t lim = std::min<size_t>((size_t)8 * g.N * p->npix, room);
-    // whole CTAs of tilts
-    auto whole = [&](int tc) { return tc < T && tc >= plan->tg ? tc - tc % plan->tg : tc; };
-    const int want = whole((int)std::min<size_t>((size_t)T, std::max<size_t>(1, lim / per_tilt)));
+    const int want = fpr_tilts_per_launch(g, *plan, T);
     int tc = want;
     if (grow && per_tilt * (size_t)tc > p->fppart_cap && !capturing(p)) {
         if (p->fpr_refused_at != g_releases.load()) p->fpr_refused = SIZE_MAX;
         size_t refused = p->fpr_refused;
-        for (int t = tc; t >= 1 && per_tilt * (size_t)t > p->fppart_cap; t = whole(t / 2)) {
+        for (int t = tc; t >= 1 && per_tilt * (size_t)t > p->fppart_cap; t = fpr_whole(*plan, T, t / 2)) {
             if (per_tilt * (size_t)t >= refused) continue;
             if (grow_fppart(p, per_tilt * (size_t)t)) break;
             refused = per_tilt * (size_t)t;
@@ -301,7 +334,7 @@ int fpr_prepare(tomo_projector* p, int T, FprPlan* plan, bool grow = true) {
         p->fpr_refused = refused;
         p->fpr_refused_at = g_releases.load();
     }
-    tc = whole((int)std::min<size_t>((size_t)want, p->fppart_cap / per_tilt));
+    tc = fpr_whole(*plan, T, (int)std::min<size_t>((size_t)want, p->fppart_cap / per_tilt));
     if (p->tilts_per_cta > 0) plan->tg = std::min({p->tilts_per_cta, kFprMaxTilts, T});
     return tc;
 }
@@ -710,6 +743,45 @@ tomo_status tomo_device_memory(uint64_t* free_bytes, uint64_t* total_bytes) {
 }
 uint64_t tomo_kernel_launches(void) { return g_launches.load(); }
 
+static void read_geom(const tomo_geom& geom, Geometry* g) {
+    g->W = geom.W;
+    g->H = geom.H;
+    g->D = geom.D;
+    g->w = geom.w;
+    g->h = geom.h;
+    g->N = geom.nproj;
+    const double dvc[3] = {(g->W - 1) / 2.0, (g->H - 1) / 2.0, (g->D - 1) / 2.0};
+    const double dpc[4] = {(g->w - 1.0) / 2, (g->h - 1.0) / 2, (g->w - 1) / 2.0, (g->h - 1) / 2.0};
+    for (int k = 0; k < 3; k++) g->vc[k] = std::isnan(geom.vol_center[k]) ? dvc[k] : geom.vol_center[k];
+    for (int k = 0; k < 4; k++) g->pc[k] = std::isnan(geom.proj_center[k]) ? dpc[k] : geom.proj_center[k];
+    g->scale = geom.scale == 0.0 ? 1.0 : geom.scale;
+}
+
+tomo_status tomo_projection_plan(const tomo_geom* geom, int32_t precision, const double* euler, int32_t update,
+                                 int64_t* out8) {
+    if (!geom || !euler || !out8) return fail(TOMO_ERR_INVALID, "null argument");
+    if (geom->W <= 0 || geom->H <= 0 || geom->D <= 0 || geom->w <= 0 || geom->h <= 0 || geom->nproj <= 0 || update < 0)
+        return fail(TOMO_ERR_INVALID, "dimensions must be positive");
+    if (precision < TOMO_PREC_FP32 || precision > TOMO_PREC_FP16) return fail(TOMO_ERR_INVALID, "unknown precision");
+    for (int k = 0; k < 8; k++) out8[k] = 0;
+    Geometry g{};
+    read_geom(*geom, &g);
+    double max_step, max_space, min_space;
+    classify_tilts(g, euler, precision, &max_step, &max_space, &min_space);
+    if (!g.separable) return TOMO_OK;
+    const int T = update == 0 ? g.N : std::min(update, g.N);
+    int ndev = 0;
+    const bool gpu = cudaGetDeviceCount(&ndev) == cudaSuccess && ndev > 0;
+    cudaGetLastError();
+    const FprPlan plan = fpr_plan(fpr_geom(g, precision, max_step, max_space, min_space), T, gpu ? device_sms() : 152);
+    if (plan.zc == 0) return TOMO_OK;
+    const int tc = fpr_tilts_per_launch(g, plan, T);
+    const int64_t v[8] = {plan.zc, plan.seg,  plan.nseg, plan.nwin,
+                          plan.pitch, plan.tg, tc, (int64_t)(sizeof(float) * plan.nseg * g.w * g.h * (size_t)tc)};
+    for (int k = 0; k < 8; k++) out8[k] = v[k];
+    return TOMO_OK;
+}
+
 tomo_status tomo_create(const tomo_geom* geom, const tomo_params* params, tomo_projector** out) {
     if (!geom || !out) return fail(TOMO_ERR_INVALID, "null argument");
     *out = nullptr;
@@ -727,17 +799,7 @@ tomo_status tomo_create(const tomo_geom* geom, const tomo_params* params, tomo_p
     }
     tomo_projector* p = new tomo_projector();
     Geometry& g = p->g;
-    g.W = geom->W;
-    g.H = geom->H;
-    g.D = geom->D;
-    g.w = geom->w;
-    g.h = geom->h;
-    g.N = geom->nproj;
-    const double dvc[3] = {(g.W - 1) / 2.0, (g.H - 1) / 2.0, (g.D - 1) / 2.0};
-    const double dpc[4] = {(g.w - 1.0) / 2, (g.h - 1.0) / 2, (g.w - 1) / 2.0, (g.h - 1) / 2.0};
-    for (int k = 0; k < 3; k++) g.vc[k] = std::isnan(geom->vol_center[k]) ? dvc[k] : geom->vol_center[k];
-    for (int k = 0; k < 4; k++) g.pc[k] = std::isnan(geom->proj_center[k]) ? dpc[k] : geom->proj_center[k];
-    g.scale = geom->scale == 0.0 ? 1.0 : geom->scale;
+    read_geom(*geom, &g);
     if (params) p->params = *params;
     if (p->params.precision < TOMO_PREC_FP32 || p->params.precision > TOMO_PREC_FP16) {
         delete p;
@@ -897,16 +959,9 @@ static tomo_status setup_geometry(tomo_projector* p) {
     Geometry& g = p->g;
     const int N = g.N;
     p->plan_gen++;
-    bool integral = true, vertical = true;
-    for (int t = 0; t < N; t++) {
-        integral = integral && tilt_is_separable(&p->euler[9 * t], g);
-        vertical = vertical && tilt_is_vertical(&p->euler[9 * t]);
-    }
-    // vertical-axis tilts run on the XZ-plane kernels; rows that are not a whole row
-    // apart (scale != 1, half-row centre offsets) blend two rows (16-bit volumes excepted)
-    const bool sep = integral || (vertical && p->vtype == kVolF32);
-    g.separable = sep;
-    g.fractional = sep && !integral;
+    classify_tilts(g, p->euler.data(), p->vtype, &p->fp_max_step, &p->fp_max_space, &p->fp_min_space);
+    p->fpr_plans.clear();
+    const bool sep = g.separable;
     if (g.fractional) {
         if (!p->d_fprow) {
             CKS(alloc_n(p, &p->d_fprow, (size_t)g.h));
@@ -938,16 +993,6 @@ static tomo_status setup_geometry(tomo_projector* p) {
             return fail(TOMO_ERR_UNSUPPORTED, "16-bit volume storage needs scale 1");
     }
     if (sep) {
-        p->fpr_plans.clear();
-        p->fp_max_step = p->fp_max_space = 0;
-        p->fp_min_space = 1e30;
-        for (int t = 0; t < N; t++) {
-            const double* R = &p->euler[9 * t];
-            const double space = 1.0 / std::fabs(R[0] * g.scale);
-            p->fp_max_step = std::max(p->fp_max_step, std::fabs(R[2] / R[0]));
-            p->fp_max_space = std::max(p->fp_max_space, space);
-            p->fp_min_space = std::min(p->fp_min_space, space);
-        }
         g.fp_row_off = (int)(g.pc[1] - g.vc[1]);
         g.bp_row_off = (int)(g.pc[3] - g.vc[1]);
         std::vector<FpTilt> ft(N);
