@@ -292,6 +292,11 @@ tomo_status tomo_profile_read(tomo_projector* p, double* out4);
  * does not run on the row-vector form. */
 tomo_status tomo_projection_plan(const tomo_geom* geom, int32_t precision, const double* euler, int32_t update,
                                  int64_t* out8);
+/* Allocates that scratch now, for updates of `update` tilts (0: all) of the loaded series and
+ * an iteration's last, smaller one; less of it while memory is short (projections then take
+ * more launches).  TOMO_ERR_NOMEM: not even one tilt's sums fit, and projections would run
+ * the one-row form. */
+tomo_status tomo_reserve_projection(tomo_projector* p, int32_t update);
 /* Tilts per forward-projection CTA (0 = automatic; tuning knob). */
 tomo_status tomo_set_tilts_per_cta(tomo_projector* p, int32_t n);
 /* Volume rows per backprojection thread (tuning knob, no counterpart in the reference):

@@ -83,3 +83,14 @@ def test_a_plan_takes_microseconds(engine):
         call()
         best = min(best, time.perf_counter() - t)
     assert best < 60e-6, best
+
+
+def test_request_bytes_count_the_projectors_scratch(engine):
+    from tomoj_gb300.serving import SIRT, WBP, Request, request_bytes
+    angles = np.linspace(-60, 60, 41)
+    series = np.lib.stride_tricks.as_strided(np.zeros(1, np.float32), (41, 256, 512), (0, 0, 0))
+    wbp, sirt = [request_bytes(Request(0, 0.0, k, series, angles, 512, 256, 512)) for k in (WBP, SIRT)]
+    call, out = _call(engine, 512, 256, 512, 512, 256, 41, 60.0, 0, 1.0, 0)
+    call()
+    assert sirt - wbp == out[7] > 0
+    assert wbp >= 4 * (512 * 256 * 512 + 6 * 41 * 256 * 512)

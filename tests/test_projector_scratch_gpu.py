@@ -133,3 +133,32 @@ def test_iterations_under_a_limit(engine, update, use_graph):
                 hd.close()
     for v in runs.values():
         assert np.array_equal(v, runs["handle", None])
+
+
+@pytest.mark.parametrize("kind, update, precision", [("SIRT", 0, "fp32"), ("OS-SART", 7, "fp32"), ("TVM", 0, "fp32"),
+                                                     ("TVM", 0, "fp16"), ("OS-SART", 3, "bf16"), ("WBP", 0, "fp32")])
+def test_request_bytes_hold_the_footprint(engine, kind, update, precision):
+    """Admission counts what a request takes, the projector's scratch included, and the scratch is
+    there when the request is admitted: its iterations allocate nothing more."""
+    from tomoj_gb300.serving import WBP, EngineAdapter, Request, request_bytes
+    rng = np.random.default_rng(1)
+    req = Request(0, 0.0, kind, rng.random((41, 64, 256), dtype=np.float32), np.linspace(-60, 60, 41), 256, 64, 128,
+                  n_iter=2, update=update, precision=_abi.precision_code(precision))
+    eng = EngineAdapter(lanes=1)
+    base = engine.tomo_memory_in_use()
+    hd = eng.create(req)
+    try:
+        admitted = engine.tomo_memory_in_use() - base
+        if kind == WBP:
+            eng.run_wbp(hd, req)
+        else:
+            eng.set_members([hd])
+            for it in range(2):
+                eng.iterate([hd], [req], [it])
+            eng.set_members([])
+        used = engine.tomo_memory_in_use() - base
+    finally:
+        eng.destroy(hd)
+        eng.close()
+    assert used == admitted
+    assert used <= request_bytes(req) <= used * 1.05 + (1 << 20), (used, request_bytes(req))

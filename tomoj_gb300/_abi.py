@@ -115,6 +115,7 @@ SIGNATURES = {
     "tomo_set_profiling": (C.c_int32, [_P, C.c_int32]),
     "tomo_profile_read": (C.c_int32, [_P, _f64p]),
     "tomo_projection_plan": (C.c_int32, [C.POINTER(Geom), C.c_int32, _f64p, C.c_int32, C.POINTER(C.c_int64)]),
+    "tomo_reserve_projection": (C.c_int32, [_P, C.c_int32]),
     "tomo_set_tilts_per_cta": (C.c_int32, [_P, C.c_int32]),
     "tomo_set_bp_rows": (C.c_int32, [_P, C.c_int32]),
     "tomo_autotune": (C.c_int32, [_P, C.c_int32, C.c_int32, _f64p]),

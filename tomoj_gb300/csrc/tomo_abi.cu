@@ -1735,6 +1735,18 @@ tomo_status tomo_set_bp_rows(tomo_projector* p, int32_t rows) {
     return TOMO_OK;
 }
 
+tomo_status tomo_reserve_projection(tomo_projector* p, int32_t update) {
+    if (!p || update < 0) return fail(TOMO_ERR_INVALID, "bad argument");
+    CKS(need_series(p));
+    const int N = p->g.N, upd = update == 0 ? N : std::min(update, N);
+    for (int T : {upd, N - (N - 1) / upd * upd}) {
+        FprPlan plan{};
+        if (fpr_prepare(p, T, &plan) == 0 && plan.zc != 0)
+            return fail(TOMO_ERR_NOMEM, "no memory for the forward projector's scratch");
+    }
+    return TOMO_OK;
+}
+
 // Autotuner: candidate kernel shapes timed on one update of this handle's series.
 tomo_status tomo_autotune(tomo_projector* p, int32_t update, int32_t reps, double* out4) {
     if (!p || reps < 0) return fail(TOMO_ERR_INVALID, "bad argument");

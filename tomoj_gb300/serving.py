@@ -38,6 +38,7 @@ measured rates, for schedules too long to serve in a benchmark run.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import heapq
 import queue
 import threading
@@ -124,6 +125,10 @@ def lane_of(req: Request, bounds) -> int:
     return len(bounds)
 
 
+def _update(req: Request) -> int:
+    return 0 if req.kind in (SIRT, TVM) else req.update
+
+
 class EngineAdapter:
     """The engine calls the server needs (a fake with the same methods tests the scheduling
     on CPU): one batch per lane, lane 0 on the most urgent stream priority."""
@@ -138,6 +143,8 @@ class EngineAdapter:
             self.batches.append(b)
             _abi.check(self.lib.tomo_batch_set_priority(b, self.n_lanes - 1 - i))
         self.top_priority = self.n_lanes
+        self.live = 0  # handles created and not destroyed
+        self.live_lock = threading.Lock()
 
     def close(self):
         for b in self.batches:
@@ -190,9 +197,21 @@ class EngineAdapter:
                     lib.tomo_destroy(hd)
                     return None
                 _abi.check(rc)
+            if req.kind != WBP:
+                # the projector's scratch now rather than in the first iteration, so that admission
+                # sees it.  Without any the projections would take another order of sums: the request
+                # waits for memory, unless no other request can give some back.
+                rc = lib.tomo_reserve_projection(hd, _update(req))
+                if rc == _abi.ERR_NOMEM and self.live > 0:
+                    lib.tomo_destroy(hd)
+                    return None
+                if rc != _abi.ERR_NOMEM:
+                    _abi.check(rc)
         except Exception:
             lib.tomo_destroy(hd)
             raise
+        with self.live_lock:
+            self.live += 1
         return hd
 
     def run_wbp(self, hd, req: Request):
@@ -205,7 +224,7 @@ class EngineAdapter:
     def iterate(self, handles, reqs, iteration, lane: int = 0):
         M = len(handles)
         relax = np.ascontiguousarray([r.relax for r in reqs], np.float64)
-        upd = np.ascontiguousarray([0 if r.kind in (SIRT, TVM) else r.update for r in reqs], np.int32)
+        upd = np.ascontiguousarray([_update(r) for r in reqs], np.int32)
         first = np.ascontiguousarray([self.lib.tomo_first_index(r.seed, it, len(r.angles))
                                       for r, it in zip(reqs, iteration)], np.int32)
         err = np.zeros((M, 5))
@@ -221,6 +240,8 @@ class EngineAdapter:
 
     def destroy(self, hd):
         self.lib.tomo_destroy(hd)
+        with self.live_lock:
+            self.live -= 1
 
 
 class Server:
@@ -546,17 +567,40 @@ class CostModel:
         return req.series.shape[0] * req.series.shape[1] * req.series.shape[2] * 4 / self.h2d_bytes_per_s
 
 
+@functools.lru_cache(maxsize=4096)
+def _projection_scratch(W: int, H: int, D: int, w: int, h: int, angles: tuple, precision: int, update: int) -> int:
+    """Bytes of the forward projector's scratch for updates of `update` tilts (0: all) and the
+    iteration's last, smaller one."""
+    n = len(angles)
+    upd = min(update, n) if update > 0 else n
+    try:
+        lib = _abi.load()
+    except RuntimeError:  # not built: the engine's bound
+        return min(8 * n * w * h * 4, max(1 << 30, W * H * D * 2))
+    g = _abi.make_geom(W, H, D, w, h, n)
+    eul = np.ascontiguousarray([euler_angles_to_matrix(0.0, a, -0.0) for a in angles], np.float64)
+    need = 0
+    for T in {upd, n - (n - 1) // upd * upd}:
+        out = np.zeros(8, np.int64)
+        _abi.check(lib.tomo_projection_plan(C.byref(g), precision, _abi.ptr(eul, C.c_double), T,
+                                            _abi.ptr(out, C.c_int64)))
+        need = max(need, int(out[7]))
+    return need
+
+
 def request_bytes(req: Request) -> int:
     """Device bytes of a request's handle, as the engine allocates them (volume in its storage
-    type, the series, three projection-sized work buffers, the per-tilt tables; a TVM
-    request adds its TV scratch: six FP32 volumes of dual variables, and an FP32 copy of a
-    16-bit volume)."""
+    type, the series, its aligned copy, four projection-sized work buffers, the per-tilt tables; an
+    iterative request adds the forward projector's scratch, a TVM request its TV scratch: six FP32
+    volumes of dual variables, and an FP32 copy of a 16-bit volume)."""
     N, h, w = req.series.shape
     nvox = req.W * req.H * req.D
     red = req.precision != _abi.PREC_FP32
     vol = nvox * (2 if red else 4)
     tv = nvox * 4 * (7 if red else 6) if req.kind == TVM else 0
-    return vol + tv + 4 * N * h * w * 4 + 64 * N * w
+    fp = 0 if req.kind == WBP else _projection_scratch(req.W, req.H, req.D, w, h, tuple(map(float, req.angles)),
+                                                       req.precision, _update(req))
+    return vol + tv + fp + 6 * N * h * w * 4 + 64 * N * w + 8 * N * h
 
 
 def simulate(requests: list[Request], cost: CostModel, max_active: int = 64, lane_bounds=DEFAULT_LANE_BOUNDS,
