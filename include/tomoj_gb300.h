@@ -247,8 +247,8 @@ tomo_status tomo_cancel(tomo_projector* p);
  * member, then one residual reduction and one backprojection launch.  Members
  * keep their own volumes, series and options (TVM, positivity...); the batch
  * only references them, so destroy the batch before its handles.  A step's
- * launches are captured as one CUDA graph and replayed while the membership
- * and update sizes are unchanged.  Members must live on one device. */
+ * launches are captured as one CUDA graph and replayed while the membership,
+ * the update sizes and the members' series, geometry and options are unchanged.  Members must live on one device. */
 typedef struct tomo_batch tomo_batch;
 tomo_status tomo_batch_create(tomo_batch** out);
 tomo_status tomo_batch_destroy(tomo_batch* b);
@@ -261,8 +261,9 @@ tomo_status tomo_batch_set_priority(tomo_batch* b, int32_t priority);
 /* cudaStream_t passed as void* for the batch's work (NULL: the batch's own stream).
  * Members' own streams must be idle at each iteration, as with the batch's own stream. */
 tomo_status tomo_batch_set_stream(tomo_batch* b, void* stream);
-/* Persistent launches (no counterpart in the reference; default off): each forward phase
- * is one launch, and each backprojection phase one launch per storage type and rule set, of
+/* Persistent launches (no counterpart in the reference; default off): each forward phase is
+ * one launch (one per group of tilts whose segment sums fit the members' scratch) and the
+ * closing pass, and each backprojection phase one launch per storage type and rule set, of
  * resident CTAs that take work items from a device list, longest first, through an atomic
  * cursor.  Off: one launch per kernel variant with a CTA per item.  Results are bitwise
  * the same.  on: 0 off, 1 on; for tuning, a sum of 2 (forward phase persistent), 4
@@ -300,9 +301,10 @@ tomo_status tomo_reserve_projection(tomo_projector* p, int32_t update);
 /* Tilts per forward-projection CTA (0 = automatic; tuning knob). */
 tomo_status tomo_set_tilts_per_cta(tomo_projector* p, int32_t n);
 /* Volume rows per backprojection thread (tuning knob, no counterpart in the reference):
- * 0 = by size and storage type, 1 = one row, 2 = two rows (FP32 volumes with a vertical
- * tilt axis and whole-row centre offsets; otherwise one row).  Results are bitwise the
- * same either way. */
+ * 0 = by size and storage type, 1 = one row, 2 = two rows (vertical tilt axis and whole-row
+ * centre offsets; 16-bit volumes for updates of up to 64 tilts without NaN / Inf and
+ * positivity rules, and not in batches; otherwise one row).  Results are bitwise the same
+ * either way. */
 tomo_status tomo_set_bp_rows(tomo_projector* p, int32_t rows);
 /* Autotuner (no counterpart in the reference): times the forward projection with
  * difference and the backprojection of one update of `update` tilts (0: all) of the
@@ -312,7 +314,7 @@ tomo_status tomo_set_bp_rows(tomo_projector* p, int32_t rows);
  * the fastest on the handle (tomo_set_tilts_per_cta / tomo_set_bp_rows; batches use each
  * member's choice).  The added projections are cleared; the volume is saved and put back.
  * Every candidate computes the same values, up to the FP32 summation order where a tilt
- * grouping changes the depth split of a small grid.  out4 (may be NULL): {tilts per CTA
+ * grouping changes the depth split of a small grid on the one-row form.  out4 (may be NULL): {tilts per CTA
  * (0 = automatic), rows per thread, forward ms, backprojection ms} of the choice. */
 tomo_status tomo_autotune(tomo_projector* p, int32_t update, int32_t reps, double* out4);
 /* Failure-path test hook (no counterpart in the reference): while enabled, the

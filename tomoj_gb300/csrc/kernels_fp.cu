@@ -359,20 +359,18 @@ struct CtaGrid {
     }
     // No grid of few CTAs is faster: the mean, and the busiest SM's CTAs at the shortest times there are.
     double least() const {
-        const double end = weight(nseg - 1), other = nseg > 1 ? weight(0) : end;
-        const int rounds = (int)(((long long)nseg * per_seg + sms - 1) / sms);
-        const int ends = end < other ? std::min(per_seg, rounds) : 0;
-        return std::max(mean(), ends * end + (rounds - ends) * std::min(other, end >= other ? end : other)) * (1.0 - 1e-9);
+        const double end = weight(nseg - 1), other = nseg > 1 ? weight(0) : end;  // end <= other <= the rest
+        const int rounds = (int)(((long long)nseg * per_seg + sms - 1) / sms), ends = std::min(per_seg, rounds);
+        return std::max(mean(), ends * end + (rounds - ends) * other) * (1.0 - 1e-9);
     }
     // Few CTAs, each taken by the SM that is free first.
     double simulated() const {
         std::vector<double> free_at(sms, 0.0);  // a binary heap, earliest first
         const long long n = (long long)nseg * per_seg;
-        long long k = 0;
         double end = 0;
         for (int s = 0; s < nseg; s++) {
             const double w = weight(s);
-            for (int q = 0; q < per_seg; q++, k++) {
+            for (int q = 0; q < per_seg; q++) {
                 if (n <= sms) {  // an SM for every CTA
                     end = std::max(end, w);
                     break;

@@ -300,7 +300,7 @@ int fpr_tilts_per_launch(const Geometry& g, const FprPlan& plan, int T) {
 // The segment sums of a launch take at most eight times the series' size (the handle holds
 // six such buffers) and 1 GiB, or half the bytes of an FP32 volume where that is more (every launch
 // reads the volume again: a SIRT iteration of 2048 x 512 x 2048 with 121 tilts takes 176 ms in launches
-// of five tilts, 161 ms in launches of 24); more tilts run in further launches, which changes no
+// of five tilts, 161 ms in launches of 22); more tilts run in further launches, which changes no
 // sum.  Where memory is refused, scratch of half as many tilts is tried and so on, down to what the
 // handle holds; the one-row form is left for a handle that cannot hold one tilt's sums.  A refused
 // size is not tried again before some device memory has been given back (g_releases).  Volumes that

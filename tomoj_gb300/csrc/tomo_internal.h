@@ -134,7 +134,7 @@ struct FprPlan {
     int pitch;    // columns of a plane buffer
     int tg;       // tilts per CTA
     int rawrows;  // volume rows staged per plane (8; fractional rows: the rows eight of them touch)
-    int bulk;     // rows start on 16-byte boundaries: the first chunk comes by bulk copies
+    int bulk;     // rows start on 16-byte boundaries: chunks come by bulk copies
     int jfirst;   // projection row of the first row group
 };
 
