@@ -26,10 +26,10 @@
 // row's result does not depend on how rows, tilts or launches are grouped.
 //
 // Measured (with fp_finish) against the one-row kernel of fp_kernel.cuh: 512 x 256 x 512, 7
-// tilts 188 us (246), 41 tilts 1.04 ms (1.37); 2048 x 512 x 2048, 121 tilts 112 ms (140);
-// 333 x 67 x 150, one tilt 20 us (43).  14 samples per wavefront (8.8 there); the data path
-// is 70-75 % busy over the launch, the rest is latency of the loads at 16 warps per SM and the
-// chunk barriers.
+// evenly spread tilts 192 us, 213 us on average over the subsets of an iteration (246), 41 tilts
+// 1.04 ms (1.37); 2048 x 512 x 2048, 121 tilts 97 ms (140); 333 x 67 x 150, one tilt 20 us (43).
+// 14 samples per wavefront (8.8 there); the data path is 60 % busy over a 7-tilt launch, the
+// rest is latency of the loads at 16 warps per SM and the chunk barriers.
 #pragma once
 #include <climits>
 #include <type_traits>
