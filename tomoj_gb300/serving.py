@@ -342,9 +342,9 @@ class Server:
                         return
                     if hd is None:  # HBM short for this head: try the next lane
                         slots[li].release()
-                        with lock:
-                            alone = inflight[0] == 0
-                        if alone:  # nothing running will free memory: the request can never fit
+                        # nothing was running that could free memory (a completion since the attempt
+                        # may have made the room that it lacked): the request can never fit
+                        if alone:
                             fail(_abi.NoMemoryError(-3, f"request {req.rid} does not fit in free HBM"))
                             return
                         continue
